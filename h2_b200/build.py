@@ -10,14 +10,16 @@ import os
 import shutil
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libh2g.so")
 # (source, extra flags): the model builder is compiled without FMA contraction
-SOURCES = [("h2g_solver.cu", []), ("h2g_model.cu", ["-fmad=false"]), ("h2g_noalloc.cu", [])]
-DEPS = ["h2g_internal.cuh", "h2g_kernels.cuh", "h2g_sweep.cuh", "h2g_multi.cuh", "h2g_coop.cuh", os.path.join("..", "..", "include", "h2g.h")]
+SOURCES = [("h2g_solver.cu", []), ("h2g_resident.cu", []), ("h2g_model.cu", ["-fmad=false"]), ("h2g_noalloc.cu", [])]
+DEPS = ["h2g_internal.cuh", "h2g_device.cuh", "h2g_kernels.cuh", "h2g_sweep.cuh", "h2g_multi.cuh", "h2g_coop.cuh",
+        "h2g_resident.cuh", os.path.join("..", "..", "include", "h2g.h")]
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
@@ -46,10 +48,14 @@ def build(force: bool = False, verbose: bool = False) -> str:
     base = [nvcc(), "-O3", "-std=c++17", *ARCH, "-lineinfo", "-Xcompiler", "-fPIC,-ffp-contract=off",
             "-I", os.path.join(ROOT, "include")]
     objs, text = [], []
+    jobs = []  # the sources compile side by side
     for src, extra in SOURCES:
         obj = os.path.join(bdir, src.replace(".cu", ".o"))
         cmd = base + extra + ["-Xptxas", "-v", "-c", os.path.join(CSRC, src), "-o", obj]
-        proc = subprocess.run(cmd, capture_output=True, text=True)
+        jobs.append((src, obj, cmd))
+    with ThreadPoolExecutor(len(jobs)) as pool:
+        procs = list(pool.map(lambda j: subprocess.run(j[2], capture_output=True, text=True), jobs))
+    for (src, obj, cmd), proc in zip(jobs, procs):
         text.append(" ".join(cmd) + "\n" + proc.stdout + proc.stderr)
         if proc.returncode != 0:
             open(log, "w").write("\n".join(text))

@@ -22,17 +22,6 @@ struct GridBar {
   unsigned int gen;
 };
 
-__device__ __forceinline__ unsigned int ld_relaxed_u32(const unsigned int* p) {
-  unsigned int v;
-  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ int ld_relaxed_s32(const int* p) {
-  int v;
-  asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
 // All blocks of the grid meet here.  Returns false (in every thread of the block) when the
 // barrier gave up: this block's wait ran out (it then sets *err and stops the solve) or another
 // block's did.  st (may be null) receives the stop.  One thread per block arrives and polls; it

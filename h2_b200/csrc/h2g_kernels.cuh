@@ -10,7 +10,7 @@
 // it once per solve in exactly the reference's operation order; the kernels look it up.
 // FP64 results are therefore bit-identical to the reference's per-cell arithmetic.
 #pragma once
-#include "h2g_internal.cuh"
+#include "h2g_device.cuh"
 
 namespace h2g {
 
@@ -18,9 +18,6 @@ namespace h2g {
 // dot products, and with it the iteration count, so it stays at 8 unless rebuilt on purpose.
 // H2G_MINB = 4 resident colour-pass blocks per SM caps that kernel at 64 registers (measured
 // 1% faster per iteration than the unconstrained 80 on the 240x240x30 grid).
-#ifndef H2G_BY
-#define H2G_BY 8
-#endif
 #ifndef H2G_MINB
 #define H2G_MINB 4
 #endif
@@ -51,10 +48,6 @@ namespace h2g {
 #ifndef H2G_AX_MINB
 #define H2G_AX_MINB 5
 #endif
-
-constexpr int kBX = 32;       // threads along the half-row
-constexpr int kBY = H2G_BY;   // rows per block
-constexpr int kThreads = kBX * kBY;
 
 // ------------------------------------------------------------------------------------------
 // Deterministic reductions: every block writes its partial sums; the last block to finish
@@ -92,118 +85,6 @@ __device__ __forceinline__ void pdl_enter() {
 
 __device__ __forceinline__ void set_cond(cudaGraphConditionalHandle h, int use_cond, int value) {
   if (use_cond) cudaGraphSetConditional(h, value ? 1u : 0u);
-}
-
-// Scalar logic of each stage (runs on one thread).  Mirrors the control flow of PBiCGSTAB!
-// (NonUniform.jl:262-349) and CG! (NonUniform.jl:131-225).
-__device__ void finish_stage(int stage, SolverState* st, double s1, double s2) {
-  switch (stage) {
-    case kStageInit:  // NonUniform.jl:263-294: res0, early return, rho of iteration 1
-    case kStageInitCg: {
-      const double res0 = sqrt(s1);
-      st->res0 = res0;
-      st->res = 1.0;
-      st->rho = s1;
-      st->rho_old = 1.0;
-      st->alpha = 0.0;
-      st->omega = 1.0;
-      st->beta = 0.0;
-      st->itr = 1;
-      st->first = 1;
-      st->stop = 0;
-      st->converged = 0;
-      st->reason = kRunning;
-      if (res0 == 0.0) {
-        st->stop = 1; st->converged = 1; st->itr = 0; st->res = 0.0; st->reason = kConverged;
-      } else if (!isfinite(res0)) {
-        st->stop = 1; st->itr = 0; st->reason = kNonFinite;
-      } else if (stage == kStageInit && fabs(s1) < kFloatMin) {
-        st->stop = 1; st->reason = kBreakdown;
-      }
-      break;
-    }
-    case kStageAlpha:  // NonUniform.jl:309
-      st->alpha = __ddiv_rn(st->rho, s1);
-      break;
-    case kStageOmega:  // NonUniform.jl:320-326
-      if (fabs(s1) < kFloatMin) { st->stop = 1; st->reason = kBreakdown; }
-      else st->omega = __ddiv_rn(s2, s1);
-      break;
-    case kStageUpdate: {  // NonUniform.jl:331-346 and the top of the next iteration 289-299
-      const double res = __ddiv_rn(sqrt(s1), st->res0);
-      if (st->hist && st->itr >= 1 && st->itr <= st->hist_len) st->hist[st->itr - 1] = res;
-      st->res = res;
-      st->first = 0;
-      if (res < st->tol) { st->stop = 1; st->converged = 1; st->reason = kConverged; break; }
-      if (!isfinite(res) || (st->div_limit > 0.0 && res > st->div_limit)) {
-        st->stop = 1; st->reason = kNonFinite; break;
-      }
-      if (st->itr >= st->maxItr) { st->stop = 1; st->reason = kMaxItr; break; }
-      st->rho_old = st->rho;
-      st->rho = s2;
-      st->itr += 1;
-      if (fabs(s2) < kFloatMin) { st->stop = 1; st->reason = kBreakdown; break; }
-      st->beta = __ddiv_rn(__dmul_rn(__ddiv_rn(st->rho, st->rho_old), st->alpha), st->omega);
-      break;
-    }
-    case kStageResid:
-      st->scale = sqrt(s1);
-      break;
-    case kStageCgInit:  // NonUniform.jl:155
-      st->rho_old = s1;
-      st->itr = 1;
-      break;
-    case kStageCgAlpha:  // NonUniform.jl:168-176
-      if (fabs(s1) < kFloatMin) { st->stop = 1; st->reason = kBreakdown; }
-      else st->alpha = __ddiv_rn(st->rho_old, s1);
-      break;
-    case kStageCgRes: {  // NonUniform.jl:185-198
-      const double res = __ddiv_rn(sqrt(s1), st->res0);
-      if (st->hist && st->itr >= 1 && st->itr <= st->hist_len) st->hist[st->itr - 1] = res;
-      st->res = res;
-      if (res < st->tol) { st->stop = 1; st->converged = 1; st->reason = kConverged; break; }
-      if (!isfinite(res) || (st->div_limit > 0.0 && res > st->div_limit)) { st->stop = 1; st->reason = kNonFinite; }
-      break;
-    }
-    case kStageCgBeta:  // NonUniform.jl:206-222, then the loop bound
-      if (fabs(s1) < kFloatMin) { st->stop = 1; st->reason = kBreakdown; break; }
-      st->beta = __ddiv_rn(s1, st->rho_old);
-      st->rho_old = s1;
-      if (st->itr >= st->maxItr) { st->stop = 1; st->reason = kMaxItr; break; }
-      st->itr += 1;
-      break;
-    case kStageDot:
-      st->dot1 = s1;
-      st->dot2 = s2;
-      break;
-    case kStageSorInit: {  // solveSOR! NonUniform.jl:1031-1035: res0 (1 if zero)
-      double res0 = sqrt(s1);
-      if (res0 == 0.0) res0 = 1.0;
-      st->res0 = res0;
-      st->res = 1.0;
-      st->itr = 0;
-      st->stop = 0;
-      st->converged = 0;
-      st->reason = kRunning;
-      if (!isfinite(res0)) { st->stop = 1; st->reason = kNonFinite; }
-      break;
-    }
-    case kStageSorHalf:  // colour 0 of rbsor! (NonUniform.jl:952-955)
-      st->dot1 = s1;
-      break;
-    case kStageSorIter: {  // colour 1, then the test of solveSOR! (NonUniform.jl:1038-1048)
-      const double res = __ddiv_rn(sqrt(__dadd_rn(st->dot1, s1)), st->res0);
-      st->itr += 1;
-      if (st->hist && st->itr <= st->hist_len) st->hist[st->itr - 1] = res;
-      st->res = res;
-      if (res < st->tol) { st->stop = 1; st->converged = 1; st->reason = kConverged; break; }
-      if (!isfinite(res)) { st->stop = 1; st->reason = kNonFinite; break; }
-      if (st->itr >= st->maxItr) { st->stop = 1; st->reason = kMaxItr; break; }
-      break;
-    }
-    default:
-      break;
-  }
 }
 
 // COND: the kernel may set the loop condition of a device-side WHILE node.  Kernels compiled
@@ -317,11 +198,10 @@ __device__ __forceinline__ bool cell_coef(const OpParams<T>& op, int k, uint8_t 
 // every value is the one cell_coef gives the cell; a cell then reads a 2-byte class index and one
 // 64-byte row instead of the 8-byte key word, six table entries and dd.  A transient grid adds
 // a_p0 per cell, so there dd is read from the per-cell array (the same value again).
-constexpr unsigned kNoClass = 0xffffu;
 constexpr int kClassSlots = 1 << 17;   // hash slots of the (plane, keys) pairs
 constexpr int kMaxClasses = 65535;     // class indices are 16-bit; 0xffff marks "not updated"
 
-// Row layout (8 values of T): cx-, cx+, cy-, cy+, cz-, cz+, dd, 0.  The FP32 rows serve the FP32
+// Row layout (8 values of T): cx-, cx+, cy-, cy+, cz-, cz+, dd, RN(1/dd) (FP64; 0 in FP32).  The FP32 rows serve the FP32
 // smoother only (its CalcAX uses the difference form, which needs a per-cell term the row lacks).
 template <typename T>
 __device__ __forceinline__ bool class_coef(const OpParams<T>& op, unsigned cl, int ci, Coef<T>& c) {
@@ -420,8 +300,6 @@ __device__ __forceinline__ T apply_a(const Coef<T>& c, T x0, T xp, T xm, T yp, T
 // both colours of its column at plane k.  All loads of a thread are issued before its first
 // store.  Offsets are 32-bit.
 // ------------------------------------------------------------------------------------------
-constexpr unsigned kFull = 0xffffffffu;
-
 template <typename T>
 __device__ __forceinline__ T ldro(const T* p) { return __ldg(p); }
 // Loads of a vector that this launch itself writes (the cooperative preconditioner, whose passes
@@ -1528,7 +1406,7 @@ __global__ void __launch_bounds__(256) k_class_assign(Geo g, const unsigned long
 // the class gets), in the precision of the tables op points to.
 template <typename T>
 __global__ void __launch_bounds__(128) k_class_coef(OpParams<T> op, const unsigned long long* __restrict__ words,
-                                                     int ncls, T* __restrict__ ctab) {
+                                                     int ncls, T* __restrict__ ctab, int* no_recip) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ncls) return;
   const unsigned long long w = words[c];
@@ -1546,6 +1424,11 @@ __global__ void __launch_bounds__(128) k_class_coef(OpParams<T> op, const unsign
   t[5] = cf.czp;
   t[6] = cf.dd;
   t[7] = T(0);
+  if constexpr (sizeof(T) == 8) {
+    // RN(1/dd) for the quotients of the resident preconditioner, which needs dd within 2^+-100
+    t[7] = __ddiv_rn(1.0, cf.dd);
+    if (!(cf.dd >= 0x1p-100 && cf.dd <= 0x1p100)) atomicExch(no_recip, 1);
+  }
 }
 
 // ------------------------------------------------------------------------------------------

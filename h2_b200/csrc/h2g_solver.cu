@@ -14,6 +14,7 @@
 #include <atomic>
 #include <map>
 #include <cmath>
+#include <condition_variable>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -29,6 +30,7 @@
 #include "h2g_sweep.cuh"
 #include "h2g_multi.cuh"
 #include "h2g_coop.cuh"
+#include "h2g_resident.cuh"
 
 namespace h2g {
 
@@ -95,6 +97,13 @@ struct OpTables {
   int pcap = 0;
 };
 
+// How k_resident splits the grid: R rows and np pairs of planes of a warp, nxb x ntj tiles (R = 0: unused).
+struct ResidentPlan {
+  int R = 0, np = 0, nxb = 0, ntj = 0, ntab = 0;
+  int blocks() const { return nxb * ntj; }
+  int threads(int NZ) const { return 32 * ((NZ + 2 * np - 1) / (2 * np)); }
+};
+
 struct Solver {
   Geo g{};
   int precision = H2G_FP64;
@@ -152,7 +161,7 @@ struct Solver {
   size_t partials_cap = 0;
   double* hist = nullptr;
   int hist_cap = 0;
-  SolveGraph graphs[kGNum][2];
+  SolveGraph graphs[kGNum][3];  // smoother none, gs, gs with the resident preconditioner
   // mixed-precision refinement settings
   double inner_tol = 1e-4;
   int max_outer = 40;
@@ -199,6 +208,20 @@ struct Solver {
   GridBar* gbar = nullptr;
   long long wait_limit = kWaitCycles;  // budget of one bounded wait (clock cycles)
   std::map<std::pair<const void*, int>, CUtensorMap> xmaps;  // TMA maps of x buffers (pointer, bytes/element)
+  // resident preconditioner (k_resident): the split used by the call in progress and its buffers
+  ResidentPlan rs;
+  bool tuning_forced = false;  // h2g_set_tuning asked for a launch shape of the colour passes
+  bool recip_ok = false;       // every dd of the class table is in the range of div_by
+  ulonglong2* rs_box = nullptr;
+  ulonglong2* rs_rowsum = nullptr;
+  size_t rs_box_cap = 0, rs_rowsum_cap = 0;
+  RsCtl* rs_ctl = nullptr;
+  uint16_t* rs_lcls = nullptr;  // per cell: class in its tile's numbering; per tile: its classes, their number
+  uint16_t* rs_list = nullptr;
+  int* rs_count = nullptr;
+  int rs_ntab = 0;              // rows of the largest tile table (0: to be made)
+  size_t rs_smem = 0;
+  bool rs_fits = false;
   // K right-hand sides on the handle's operator (h2g_create_multi): stacked vectors, K states
   int nrhs = 0;
   double* mr_th = nullptr;
@@ -428,6 +451,13 @@ static int sweep_status(Solver* s) {
   if (!e) return H2G_OK;
   CK(cudaMemset(s->sweep_err, 0, sizeof(int)));
   CK(cudaMemset(s->gbar, 0, sizeof(GridBar)));
+  if (s->rs_ctl) {
+    // no message of the launch that gave up may look like one of a later launch
+    const RsCtl c{1ull, 0u, 0u};
+    CK(cudaMemset(s->rs_box, 0, s->rs_box_cap));
+    CK(cudaMemset(s->rs_rowsum, 0, s->rs_rowsum_cap));
+    CK(cudaMemcpy(s->rs_ctl, &c, sizeof c, cudaMemcpyHostToDevice));
+  }
   return fail(H2G_TIMEOUT, "a bounded wait of the RB-GS preconditioner ran out");
 }
 
@@ -474,6 +504,163 @@ static int launch_coop(Solver* s, cudaStream_t cs, const OpParams<double>& op, d
                 : m == 1 ? launch_coop_np<VM, 2, 1>(s, cs, op, xx, v, r, q, st)
                          : launch_coop_np<VM, 2, 0>(s, cs, op, xx, v, r, q, st);
 }
+// ---- resident preconditioner (k_resident) ------------------------------------------------------
+const void* resident_kernel(int R, int np, int vm);
+cudaError_t launch_tile_classes(cudaStream_t st, const Geo& g, const uint16_t* cls, uint16_t* lcls, uint16_t* list,
+                                int* count, int R, int nxb, int ntj);
+static bool resident_b_shared(const ResidentPlan& pl) { return pl.R <= (pl.np == 1 ? 5 : 2); }
+
+// SMs of each device held by launches whose blocks wait for one another (k_resident, k_precond_coop).
+// Two of them that together need more blocks than the device holds could each keep the other's last
+// blocks from starting, so a call takes its SMs here first and gives them back when it is done.
+// Calls are served in order of arrival.
+struct SmPool {
+  std::mutex mu;
+  std::condition_variable cv;
+  int used = 0;
+  unsigned long long next = 0, serving = 0;
+};
+constexpr int kMaxDevices = 64;
+static SmPool g_sm_pool[kMaxDevices];
+
+class SmLease {
+ public:
+  SmLease() = default;
+  SmLease(const SmLease&) = delete;
+  SmLease& operator=(const SmLease&) = delete;
+  ~SmLease() {
+    if (!n_) return;
+    std::lock_guard<std::mutex> lk(pool_->mu);
+    pool_->used -= n_;
+    pool_->cv.notify_all();
+  }
+  void take(const Solver* s, int n) {
+    pool_ = &g_sm_pool[s->device];
+    std::unique_lock<std::mutex> lk(pool_->mu);
+    const unsigned long long mine = pool_->next++;
+    pool_->cv.wait(lk, [&] { return pool_->serving == mine && pool_->used + n <= s->num_sms; });
+    pool_->serving += 1;
+    pool_->used += n;
+    n_ = n;
+    pool_->cv.notify_all();
+  }
+
+ private:
+  SmPool* pool_ = nullptr;
+  int n_ = 0;
+};
+
+// The split of k_resident for a grid, if it has one: tiles of 32 positions x R rows x all planes with
+// the fewest rows (the shortest pass) for which there is an SM for every tile.  A warp has one pair of
+// planes up to 30 planes (up to 8 rows: 240x240x30 takes 7, 140 tiles), two pairs up to 60 planes (4
+// rows).  Larger grids keep the separate launches, as do the grids without a class table or with tiles of
+// too many classes (resident_prepare), the FP32 smoother, and handles on which a launch shape, a
+// coefficient source or another form of the preconditioner was asked for.
+static ResidentPlan resident_plan(const Solver* s) {
+  ResidentPlan no, pl;
+  const Geo& g = s->g;
+  if (s->precision != H2G_FP64 || !s->cls_ok || !s->recip_ok || !s->steady || s->nrhs) return no;
+  if (s->tuning_forced || s->sweep_forced >= 0 || s->coop_forced >= 0 || s->device >= kMaxDevices) return no;
+  for (const char* e : {"H2G_RB_ROWS", "H2G_RB_PLANES", "H2G_RB_DD", "H2G_AX_DD", "H2G_RB_FUSED", "H2G_SW_CHUNKS",
+                        "H2G_SW_DD", "H2G_RB_COOP"})
+    if (getenv(e)) return no;
+  pl.np = g.NZ <= 2 * kRsMaxWarps ? 1 : 2;
+  if (g.NZ > 4 * kRsMaxWarps) return no;
+  pl.nxb = (g.HN + 31) / 32;
+  for (pl.R = 1; pl.R <= (pl.np == 1 ? kRsMaxRows : 4); ++pl.R) {
+    pl.ntj = (g.NY + pl.R - 1) / pl.R;
+    if (pl.blocks() <= s->num_sms) return pl;
+  }
+  return no;
+}
+
+// Buffers, the tiles' own class numbers and the shared-memory attributes for the split pl.  pl.R = 0 on
+// return: a tile has more classes than fit beside its x and b.
+static int resident_prepare(Solver* s, ResidentPlan& pl) {
+  const Geo& g = s->g;
+  const size_t box = sizeof(ulonglong2) * ((size_t)pl.blocks() * ((g.NZ + 1) & ~1) * 2 * kRsBox + kRsZero);
+  if (!s->rs_ctl) {
+    const size_t nb = (size_t)pl.nxb * ((g.NY + kBY - 1) / kBY) * g.NZ;
+    CK(cudaMalloc(&s->rs_box, box));
+    CK(cudaMemset(s->rs_box, 0, box));
+    s->rs_box_cap = box;
+    s->rs_rowsum_cap = sizeof(ulonglong2) * 2 * nb * 8;
+    CK(cudaMalloc(&s->rs_rowsum, s->rs_rowsum_cap));
+    CK(cudaMemset(s->rs_rowsum, 0, s->rs_rowsum_cap));
+    CK(cudaMalloc(&s->rs_lcls, sizeof(uint16_t) * (size_t)g.n));
+    CK(cudaMemset(s->rs_lcls, 0, sizeof(uint16_t) * (size_t)g.n));
+    CK(cudaMalloc(&s->rs_list, sizeof(uint16_t) * (size_t)pl.blocks() * kRsMaxTab));
+    CK(cudaMalloc(&s->rs_count, sizeof(int) * (size_t)pl.blocks()));
+    RsCtl* c = nullptr;
+    CK(cudaMalloc(&c, sizeof(RsCtl)));
+    const RsCtl init{1ull, 0u, 0u};
+    if (cudaMemcpy(c, &init, sizeof init, cudaMemcpyHostToDevice) != cudaSuccess) {
+      cudaFree(c);
+      return fail(H2G_CUDA_ERROR, "initialising the resident preconditioner failed");
+    }
+    s->rs_ctl = c;
+    s->rs_ntab = 0;
+  }
+  if (!s->rs_ntab) {  // the classes were built anew
+    std::vector<int> count(pl.blocks());
+    CK(launch_tile_classes(s->stream, g, s->cls, s->rs_lcls, s->rs_list, s->rs_count, pl.R, pl.nxb, pl.ntj));
+    CK(cudaMemcpyAsync(count.data(), s->rs_count, sizeof(int) * count.size(), cudaMemcpyDeviceToHost, s->stream));
+    CK(cudaStreamSynchronize(s->stream));
+    s->rs_ntab = 1 + *std::max_element(count.begin(), count.end());
+    s->rs_smem = rs_smem(pl.R, g.NZ, s->rs_ntab, resident_b_shared(pl));
+    int most = 0;
+    CK(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device));
+    s->rs_fits = s->rs_ntab <= kRsMaxTab && s->rs_smem + 512 <= (size_t)most;
+    if (s->rs_fits)
+      for (int vm = 0; vm < 3; ++vm)
+        CK(cudaFuncSetAttribute(resident_kernel(pl.R, pl.np, vm), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                most - 512));
+  }
+  pl.ntab = s->rs_ntab;
+  if (!s->rs_fits) pl.R = 0;
+  return H2G_OK;
+}
+
+static int launch_resident(Solver* s, cudaStream_t cs, const OpParams<double>& op, int vm, double* xx, double* v,
+                           const double* r, const double* q, double* y, const double* u, SolverState* st) {
+  RsArgs a;
+  a.op = op;
+  a.xx = xx;
+  a.v = v;
+  a.r = r;
+  a.q = q;
+  a.y = y;
+  a.u = u;
+  a.st = st;
+  a.rowsum = s->rs_rowsum;
+  a.partials = s->partials;
+  a.box = s->rs_box;
+  a.ctl = s->rs_ctl;
+  a.lcls = s->rs_lcls;
+  a.list = s->rs_list;
+  a.count = s->rs_count;
+  a.ntab = s->rs.ntab;
+  a.err = s->sweep_err;
+  a.limit = s->wait_limit;
+  a.nxb = s->rs.nxb;
+  a.ntj = s->rs.ntj;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(s->rs.blocks());
+  cfg.blockDim = dim3(s->rs.threads(op.g.NZ));
+  cfg.dynamicSmemBytes = s->rs_smem;
+  cfg.stream = cs;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  void* args[] = {&a};
+  if (cudaLaunchKernelExC(&cfg, resident_kernel(s->rs.R, s->rs.np, vm), args) != cudaSuccess)
+    return fail(H2G_CUDA_ERROR, "cooperative launch of %d blocks failed: %s", s->rs.blocks(),
+                cudaGetErrorString(cudaGetLastError()));
+  return H2G_OK;
+}
+
 static bool use_coop(const Solver* s) { return s->rb_coop && !s->coop_barred && !s->rb_fused; }
 
 template <typename T>
@@ -530,6 +717,7 @@ static int launch_precond(Solver* s, cudaStream_t cs, const OpParams<T>& op, T* 
   // k_rb_first updates v in place (VM 1 reads and writes p there)
   TV* v = VM == 0 ? vin : vout;
   if constexpr (std::is_same<T, double>::value && std::is_same<TV, double>::value) {
+    if (VM == 0 && s->rs.R && !none) return launch_resident(s, cs, op, 0, xx, v, nullptr, nullptr, nullptr, nullptr, st);
     if (use_coop(s) && !none && !bbT) return launch_coop<VM>(s, cs, op, xx, v, r, q, st);
   }
   if (s->rb_cls && op.cls && !none)
@@ -639,6 +827,8 @@ static void destroy(Solver* s) {
   cudaFree(s->x2_64); cudaFree(s->x2_32); cudaFree(s->sweep_err); cudaFree(s->gbar);
   cudaFree(s->cls); cudaFree(s->ctab); cudaFree(s->ctab32); cudaFree(s->cslots); cudaFree(s->slot_class); cudaFree(s->cwords);
   cudaFree(s->cflag); cudaFree(s->key_prev); cudaFree(s->kdiff);
+  cudaFree(s->rs_box); cudaFree(s->rs_rowsum); cudaFree(s->rs_ctl); cudaFree(s->rs_lcls); cudaFree(s->rs_list);
+  cudaFree(s->rs_count);
   s->mr_graph.reset();
   cudaFree(s->mr_th); cudaFree(s->mr_b); cudaFree(s->mr_st); cudaFree(s->mr_ctl); cudaFree(s->mr_partials);
   cudaFree(s->mr_flag);
@@ -697,6 +887,7 @@ static int build_classes(Solver* s) {
   const bool was = s->cls_ok;
   s->cls_ok = false;
   s->ncls = 0;
+  s->rs_ntab = 0;
   const char* e = getenv("H2G_CLS");
   if ((e && atoi(e) == 0) || g.NZ > 255 || !s->nkey) {
     if (was) invalidate_graphs(s);
@@ -744,14 +935,17 @@ static int build_classes(Solver* s) {
   k_class_assign<<<gi, 256, 0, s->stream>>>(g, s->nkey, s->cslots, s->slot_class, s->cls);
   const int ncls = (int)words.size();
   OpParams<double> o64 = op_params_rc<double>(s, s->t64, s->rc64);
-  k_class_coef<double><<<(ncls + 127) / 128, 128, 0, s->stream>>>(o64, s->cwords, ncls, s->ctab);
+  CK(cudaMemsetAsync(s->cflag, 0, sizeof(int), s->stream));
+  k_class_coef<double><<<(ncls + 127) / 128, 128, 0, s->stream>>>(o64, s->cwords, ncls, s->ctab, s->cflag);
   if (s->ctab32) {
     OpParams<float> o32 = op_params_rc<float>(s, s->t32, s->rc32);
-    k_class_coef<float><<<(ncls + 127) / 128, 128, 0, s->stream>>>(o32, s->cwords, ncls, s->ctab32);
+    k_class_coef<float><<<(ncls + 127) / 128, 128, 0, s->stream>>>(o32, s->cwords, ncls, s->ctab32, nullptr);
   }
   CKL();
+  CK(cudaMemcpyAsync(&flag, s->cflag, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));  // the host vectors must outlive the copies
   s->ncls = ncls;
+  s->recip_ok = flag == 0;
   s->cls_ok = true;
   if (!was) invalidate_graphs(s);
   return H2G_OK;
@@ -919,6 +1113,24 @@ static int launch_pbicg_body(Solver* s, cudaStream_t cs, const OpParams<T>& opA,
   T* t = kvec<T>(s, KT);
   TP* bbm = std::is_same<T, TP>::value ? nullptr : kvec<TP>(s, KBB);
   TP* x2 = x2buf<TP>(s);
+  auto launch_update = [&] {
+    // x += alpha p_ + omega s_; r = s - omega t; res; next rho    NonUniform.jl:328-346
+    if (use_cond)
+      launch(s, k_bicg_update<T, TX, TP, true>, elementwise_blocks(s), 256, cs, g.n, x, ph, sh, r, sv, t, r0, st,
+             s->partials, hc, use_cond);
+    else
+      launch(s, k_bicg_update<T, TX, TP, false>, elementwise_blocks(s), 256, cs, g.n, x, ph, sh, r, sv, t, r0, st,
+             s->partials, hc, use_cond);
+  };
+  if constexpr (std::is_same<T, double>::value && std::is_same<TP, double>::value) {
+    if (s->rs.R && smoother != H2G_SMOOTHER_NONE) {
+      // the same steps: p, p_ and q = A p_ with alpha; s, s_ and t = A s_ with omega
+      if (int rc = launch_resident(s, cs, opM, 1, ph, p_out, r, q, q, r0, st)) return rc;
+      if (int rc = launch_resident(s, cs, opM, 2, sh, sv, r, q, t, nullptr, st)) return rc;
+      launch_update();
+      return H2G_OK;
+    }
+  }
   // p = r + beta (p - omega q); p_ = M^-1 p                     NonUniform.jl:296-305
   if (int rc = launch_precond<TP, T, 1>(s, cs, opM, ph, x2, p_in, p_out, bbm, r, q, st, smoother)) return rc;
   // q = A p_;  alpha = rho / (q, r0)                            NonUniform.jl:307-309
@@ -927,13 +1139,7 @@ static int launch_pbicg_body(Solver* s, cudaStream_t cs, const OpParams<T>& opA,
   if (int rc = launch_precond<TP, T, 2>(s, cs, opM, sh, x2, sv, sv, bbm, r, q, st, smoother)) return rc;
   // t = A s_; omega = (t,s)/(t,t)                               NonUniform.jl:317-326
   launch_ax<T, 2, TP>(s, cs, opA, t, sh, nullptr, sv, st, kStageOmega);
-  // x += alpha p_ + omega s_; r = s - omega t; res; next rho    NonUniform.jl:328-346
-  if (use_cond)
-    launch(s, k_bicg_update<T, TX, TP, true>, elementwise_blocks(s), 256, cs, g.n, x, ph, sh, r, sv, t, r0, st,
-           s->partials, hc, use_cond);
-  else
-    launch(s, k_bicg_update<T, TX, TP, false>, elementwise_blocks(s), 256, cs, g.n, x, ph, sh, r, sv, t, r0, st,
-           s->partials, hc, use_cond);
+  launch_update();
   return H2G_OK;
 }
 
@@ -1038,9 +1244,16 @@ static int make_loop_graph(Solver* s, SolveGraph& G, Body body) {
 template <typename T, typename TX, typename TP>
 static int get_graph(Solver* s, int kind, int smoother, const OpParams<T>& op, const OpParams<TP>& opM, TX* x,
                      SolverState* st, SolveGraph** out) {
-  SolveGraph& G = s->graphs[kind][smoother ? 1 : 0];
+  const bool resident = std::is_same<T, double>::value && std::is_same<TP, double>::value && s->rs.R && smoother;
+  SolveGraph& G = s->graphs[kind][resident ? 2 : smoother ? 1 : 0];
   std::vector<unsigned char> sig = signature(op, opM, smoother, (const void*)x);
   sig.push_back(use_coop(s) ? 1 : 0);
+  if (resident) {
+    const unsigned char* d = reinterpret_cast<const unsigned char*>(&s->rs);
+    sig.insert(sig.end(), d, d + sizeof s->rs);
+    d = reinterpret_cast<const unsigned char*>(&s->rs_box);
+    sig.insert(sig.end(), d, d + sizeof s->rs_box);
+  }
   if (G.exec && G.sig == sig) {
     *out = &G;
     return H2G_OK;
@@ -1146,15 +1359,16 @@ static void print_log(const SolverState& st, const double* hist, int nhist, int 
 
 // Kernels of one preconditioner call: the first pass and 9 colour passes, or 5 fused sweeps (the
 // first one with the Krylov update).
-static int precond_kernels(const Solver* s, int smoother, bool coop = false) {
-  if (smoother == H2G_SMOOTHER_NONE || coop) return 1;
+static int precond_kernels(const Solver* s, int smoother, bool coop = false, bool resident = false) {
+  if (smoother == H2G_SMOOTHER_NONE || coop || resident) return 1;
   return s->rb_fused ? kSweeps : 2 * kSweeps;
 }
 
 // Kernels in one WHILE-body pass (one Krylov iteration); coop: the preconditioner is the one
 // cooperative launch (FP64 smoother).
-static long long body_kernels(const Solver* s, bool cg, int smoother, bool coop = false) {
-  const int pc = precond_kernels(s, smoother, coop);
+static long long body_kernels(const Solver* s, bool cg, int smoother, bool coop = false, bool resident = false) {
+  const int pc = precond_kernels(s, smoother, coop, resident);
+  if (resident && !cg) return 3;  // CalcAX runs behind the preconditioner
   return cg ? (1 + 1 + pc + 1 + 1) : (2 * pc + 2 + 1);
 }
 
@@ -1204,9 +1418,10 @@ static int solve_krylov(Solver* s, bool cg, double tol, int maxItr, int smoother
   const int nprint = (fin.reason == kBreakdown || fin.reason == kNonFinite) ? std::min(nh, std::max(0, fin.itr - 1)) : nh;
   if (verbose) print_log(fin, hh.data(), nprint, fin.converged);
   if (out) {
-    const bool coop = std::is_same<TP, double>::value && use_coop(s);
-    const long long body = body_kernels(s, cg, smoother, coop);
-    const long long pre = 2 + (cg ? precond_kernels(s, smoother, coop) + 1 : 0);
+    const bool resident = std::is_same<TP, double>::value && s->rs.R && smoother != H2G_SMOOTHER_NONE;
+    const bool coop = std::is_same<TP, double>::value && use_coop(s) && !resident;
+    const long long body = body_kernels(s, cg, smoother, coop, resident);
+    const long long pre = 2 + (cg ? precond_kernels(s, smoother, coop, resident) + 1 : 0);
     out->launches = pre + body * std::max(1, fin.itr);
     out->isconverged = fin.converged;
     out->itr = fin.itr;
@@ -1568,6 +1783,31 @@ static int solve_multi(Solver* s, double tol, int maxItr, int smoother, h2g_resu
 
 static int autotune(Solver* s);
 
+// The form of the preconditioner for one call, and the SMs it needs until the call returns: the
+// resident one where the grid has a split, else what the launch-shape tuner chose.
+struct ResidentCall {
+  Solver* s = nullptr;
+  SmLease lease;
+  int begin(Solver* solver, int smoother) {
+    s = solver;
+    ResidentPlan pl = smoother == H2G_SMOOTHER_GS ? resident_plan(s) : ResidentPlan();
+    if (pl.R)
+      if (int rc = resident_prepare(s, pl)) return rc;
+    if (pl.R) {
+      if (!s->rb_tuned) s->ax_cls = true;  // CG's CalcAX: the class table, untimed
+      lease.take(s, pl.blocks());
+      s->rs = pl;
+      return H2G_OK;
+    }
+    if (int rc = autotune(s)) return rc;
+    if (use_coop(s) && smoother == H2G_SMOOTHER_GS && s->device < kMaxDevices) lease.take(s, s->num_sms);
+    return H2G_OK;
+  }
+  ~ResidentCall() {
+    if (s) s->rs = ResidentPlan();
+  }
+};
+
 static int solve(Solver* s, bool cg, double tol, int maxItr, int smoother, int verbose, double* res_hist,
                  h2g_result* out) {
   if (!s->grid_set || !s->fields_set) return fail(H2G_BAD_ARG, "h2g_set_grid and h2g_set_fields must come first");
@@ -1576,7 +1816,8 @@ static int solve(Solver* s, bool cg, double tol, int maxItr, int smoother, int v
     return fail(H2G_BAD_ARG, "Unsupported smoother: %d. Use none (0) or gs (1)", smoother);
   if (!(tol >= 0.0) || !std::isfinite(tol)) return fail(H2G_BAD_ARG, "bad tolerance");
   CK(cudaSetDevice(s->device));
-  if (int rc = autotune(s)) return rc;
+  ResidentCall resident;
+  if (int rc = resident.begin(s, smoother)) return rc;
   int rc;
   if (s->precision == H2G_MIXED_IR) rc = solve_ir(s, cg, tol, maxItr, smoother, verbose, res_hist, out);
   else if (s->precision == H2G_MIXED) rc = solve_mixed(s, cg, tol, maxItr, smoother, verbose, res_hist, out);
@@ -2500,7 +2741,8 @@ static int precond_t(Solver* s, const double* bb, double* xx, int smoother, cons
   using namespace h2g;
   void *ha, *hb;
   int rc;
-  if ((rc = autotune(s))) return rc;  // before the hook buffers are filled: the tuner uses them
+  ResidentCall resident;  // before the hook buffers are filled: the tuner uses them
+  if ((rc = resident.begin(s, smoother))) return rc;
   if ((rc = hook_buffers(s, &ha, &hb))) return rc;
   T* xd = static_cast<T*>(ha);
   T* bd = static_cast<T*>(hb);
@@ -2853,6 +3095,7 @@ int h2g_set_tuning(h2g_solver* h, int rows, int planes) {
   Solver* s = S(h);
   if (rows == 0) {
     s->rb_tuned = false;
+    s->tuning_forced = false;
     return H2G_OK;
   }
   if (!h2g::valid_rows(rows)) return fail(H2G_BAD_ARG, "rows per block must be 2, 4, 8 or 16 (0: tune)");
@@ -2861,6 +3104,7 @@ int h2g_set_tuning(h2g_solver* h, int rows, int planes) {
   s->rb_rows = rows;
   s->rb_planes = planes;
   s->rb_tuned = true;
+  s->tuning_forced = true;
   return H2G_OK;
 }
 

@@ -1,0 +1,139 @@
+"""The resident preconditioner (k_resident: Krylov update, 10 colour passes and CalcAX with its inner
+products in one cooperative launch) against the oracle and against the separate launches.
+
+It must give exactly the bits of the separate launches: the preconditioner is compared with
+`array_equal` to the oracle for every number of rows per tile, planes per warp, ragged and one-tile
+grids, masked cells and every boundary type; whole PBiCGSTAB and CG solves equal the colour-pass solves
+(a forced launch shape selects those) bit for bit, residual history included.  A zero wait budget ends
+the solve with H2G_TIMEOUT and the handle keeps working."""
+import ctypes
+import threading
+
+import numpy as np
+import pytest
+
+import h2_b200
+from h2_b200 import _lib as L
+from conftest import mode3_model
+from test_gpu_boxes import GRIDS, box_problem
+from test_gpu_kernels import make_solver, random_interior
+
+pytestmark = pytest.mark.gpu
+
+# NX = 198..201 needs 4 tiles along the positions, so 37 tiles of rows: R = ceil(NY / 37)
+SIZES = [(40, 40, 30), (41, 37, 30), (62, 63, 30), (200, 74, 30), (199, 100, 30), (201, 140, 30), (198, 181, 30),
+         (200, 222, 30), (200, 230, 30), (254, 259, 30), (190, 290, 30), (50, 43, 60), (130, 70, 60), (129, 147, 60),
+         (126, 290, 60)]
+
+
+def launches_of(s, itr):
+    return 2 + 3 * itr
+
+
+@pytest.mark.parametrize("n", SIZES, ids=["x".join(map(str, n)) for n in SIZES])
+def test_preconditioner_bit_exact(oracle, n):
+    prob = mode3_model(oracle, n[0], n[1], n[2])
+    s = make_solver(prob)
+    bb = random_interior(prob.shape, sum(n))
+    assert np.array_equal(s.preconditioner(bb, "gs"), oracle.preconditioner(prob, bb, "gs"))
+    # quotients outside the range of the reciprocal steps: zeros, tiny, huge and subnormal numerators
+    bb *= np.random.default_rng(1).choice([0.0, -0.0, 1e-150, 1e-310, 1e150, 1.0], prob.shape)
+    assert np.array_equal(s.preconditioner(bb, "gs"), oracle.preconditioner(prob, bb, "gs"))
+    s.close()
+
+
+@pytest.mark.parametrize("grid", GRIDS, ids=["x".join(map(str, g)) for g in GRIDS])
+def test_preconditioner_boxes(oracle, grid):
+    prob = box_problem(oracle, *grid, seed=sum(grid) + 3)
+    s = make_solver(prob)
+    bb = random_interior(prob.shape, 5)
+    assert np.array_equal(s.preconditioner(bb, "gs"), oracle.preconditioner(prob, bb, "gs"))
+    s.close()
+
+
+def test_preconditioner_masked_cells(oracle):
+    prob = box_problem(oracle, 33, 31, 9, seed=22)
+    m = prob.wk["mask"]
+    inner = (slice(1, -1),) * 3
+    m[inner] = np.where(np.random.default_rng(5).uniform(size=m[inner].shape) < 0.1, 0.0, 1.0)
+    s = make_solver(prob)
+    bb = random_interior(prob.shape, 6)
+    assert np.array_equal(s.preconditioner(bb, "gs"), oracle.preconditioner(prob, bb, "gs"))
+    s.close()
+
+
+@pytest.mark.parametrize("method", ["pbicgstab", "cg"])
+@pytest.mark.parametrize("n", [(24, 20, 30), (41, 37, 30), (121, 117, 30), (200, 230, 30), (66, 50, 60)],
+                         ids=lambda n: "x".join(map(str, n)))
+def test_solve_identical(oracle, method, n):
+    prob = mode3_model(oracle, n[0], n[1], n[2])
+    cap = 20000 if n[0] < 150 else 60
+    out = []
+    for resident in (True, False):
+        s = make_solver(prob)
+        if not resident:
+            s.set_tuning(8, 2)
+        hist = np.zeros(cap)
+        st, res = s.solve(method, tol=1e-8, maxItr=cap, smoother="gs", hist=hist)
+        out.append((st, res.itr, res.res0, res.res, hist[:res.itr].copy(), s.get_theta()))
+        per = (3, 2) if method == "pbicgstab" else (5, 4)
+        assert (res.launches == per[1] + per[0] * res.itr) == resident
+        s.close()
+    assert out[0][:4] == out[1][:4]
+    assert np.array_equal(out[0][4], out[1][4]) and np.array_equal(out[0][5], out[1][5])
+
+
+def test_timeout_is_reported(oracle):
+    prob = mode3_model(oracle, 40)
+    ref = make_solver(prob)
+    st, rr = ref.solve("pbicgstab", tol=1e-8, maxItr=20000, smoother="gs")
+    assert st == 0 and rr.launches == launches_of(ref, rr.itr)
+    s = make_solver(prob)
+    s.snapshot()
+    for _ in range(2):
+        s.set_wait_limit(0)
+        res = L.Result()
+        st = L.load().h2g_pbicgstab(s.h, 1e-8, 200, 1, 0, None, ctypes.byref(res))
+        assert st == L.H2G_TIMEOUT and res.status == L.H2G_TIMEOUT and not res.isconverged
+        with pytest.raises(h2_b200.H2GError) as e:
+            s.preconditioner(random_interior(prob.shape, 1), "gs")
+        assert e.value.status == L.H2G_TIMEOUT
+        s.set_wait_limit(2_000_000_000)
+        s.snapshot(restore=True)
+        st, res = s.solve("pbicgstab", tol=1e-8, maxItr=20000, smoother="gs")
+        assert st == 0 and (res.itr, res.res) == (rr.itr, rr.res)
+        assert np.array_equal(s.get_theta(), ref.get_theta())
+    s.close()
+    ref.close()
+
+
+def test_two_threads(oracle):
+    """Two host threads solving on their own handles and streams: the calls share the SMs in turn and
+    each gives its lone solve's bits."""
+    import torch
+    prob = mode3_model(oracle, 62, 63)
+    ref = make_solver(prob)
+    _, rr = ref.solve("pbicgstab", tol=1e-8, maxItr=20000, smoother="gs")
+    th = ref.get_theta()
+    ref.close()
+    got = [None, None]
+
+    def work(q):
+        stream = torch.cuda.Stream()
+        s = make_solver(prob)
+        L.check(s.lib.h2g_set_stream(s.h, ctypes.c_void_p(stream.cuda_stream)))
+        s.snapshot()
+        for _ in range(4):
+            s.snapshot(restore=True)
+            st, res = s.solve("pbicgstab", tol=1e-8, maxItr=20000, smoother="gs")
+        got[q] = (st, res.itr, res.res, s.get_theta())
+        s.close()
+
+    ts = [threading.Thread(target=work, args=(q,)) for q in range(2)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    for g in got:
+        assert g[0] == 0 and g[1:3] == (rr.itr, rr.res)
+        assert np.array_equal(g[3], th)
