@@ -41,7 +41,7 @@ static __device__ __align__(256) double g_noalloc_scratch[kSlots];
 // operation order (no FMA contraction: __dmul_rn / __dadd_rn / __ddiv_rn).
 __device__ __forceinline__ double lam_f(double a, double b, double ma, double mb) {
   const double h = __ddiv_rn(__dmul_rn(__dmul_rn(2.0, a), b), __dadd_rn(a, b));
-  return __dmul_rn(h, __dsub_rn(2.0, trunc(__ddiv_rn(__dadd_rn(ma, mb), 2.0))));
+  return __dmul_rn(h, __dsub_rn(2.0, trunc(__dmul_rn(__dadd_rn(ma, mb), 0.5))));
 }
 
 struct Args {
@@ -52,84 +52,175 @@ struct Args {
   double* r;
 };
 
-__global__ void __launch_bounds__(kThreads) k_calcrk_rows(Args a, double* scratch) {
-  const int MX = a.MX, MY = a.MY;
-  const int row = blockIdx.x;  // interior row (j, k), j fastest
-  const int NY = MY - 2;
-  const int j = 1 + row % NY, k = 1 + row / NY;
+// Rows of one block: a thread walks up a column of them.
+constexpr int kRows = 8;
+
+// One block: kRows rows of a plane, 128 positions at a time.  What bounds it: theta, lambda, mask and b are
+// read once and r written once (70 MB at 240x240x30, 11 us of HBM), but a cell's six conductances cost 14
+// divisions, about 800 instructions.  Here 5 are left, side by side, and the next row's values are loaded
+// while a row is computed:
+//   * lambda_f(a, b) is symmetric to the last bit (2ab is exact up to its one rounding in either order), so a
+//     cell takes its left face from the lane on its left and its lower face from the row before;
+//   * the division by 2 is a product with 0.5 (exact), and the division by dz, the same for a whole plane,
+//     two of Markstein's correction steps from 1/dz (div_by; the same quotient);
+//   * a cell among six unmasked neighbours skips the convective terms, which are zero there.
+// (Keeping a conductance while its two materials stay the same runs fewer divisions but one after another in
+// a branch: slower.)
+__device__ __forceinline__ double div_by(double a, double d, double y) {
+  // P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
+  // Dev. 34, 1990.  d and y = RN(1/d) are normal; a out of 2^+-400 (or d out of 2^+-100) takes the division.
+  double q = __dmul_rn(a, y);
+  double r = __fma_rn(d, q, -a);
+  q = __fma_rn(-r, y, q);
+  r = __fma_rn(d, q, -a);
+  q = __fma_rn(-r, y, q);
+  const double aa = fabs(a), ad = fabs(d);
+  if (!(aa >= 0x1p-400 && aa <= 0x1p400 && ad >= 0x1p-100 && ad <= 0x1p100)) q = __ddiv_rn(a, d);
+  return q;
+}
+
+// What a cell reads besides itself and the row before.
+struct Row {
+  double lxp, lyp, lzm, lzp, mxm, mxp, myp, mzm, mzp, txm, txp, typ, tzm, tzp, b;
+};
+__device__ __forceinline__ Row load_row(const Args& a, long long c, int MX, long long pl) {
+  Row q;
+  q.lxp = __ldg(a.lam + c + 1);
+  q.lyp = __ldg(a.lam + c + MX);
+  q.lzm = __ldg(a.lam + c - pl);
+  q.lzp = __ldg(a.lam + c + pl);
+  q.mxm = __ldg(a.m + c - 1);
+  q.mxp = __ldg(a.m + c + 1);
+  q.myp = __ldg(a.m + c + MX);
+  q.mzm = __ldg(a.m + c - pl);
+  q.mzp = __ldg(a.m + c + pl);
+  q.txm = __ldg(a.th + c - 1);
+  q.txp = __ldg(a.th + c + 1);
+  q.typ = __ldg(a.th + c + MX);
+  q.tzm = __ldg(a.th + c - pl);
+  q.tzp = __ldg(a.th + c + pl);
+  q.b = a.b[c];
+  return q;
+}
+
+__global__ void __launch_bounds__(kThreads, 4) k_calcrk_rows(Args a, double* scratch) {
+  const int MX = a.MX, MY = a.MY, NX = MX - 2, NY = MY - 2, NZ = a.MZ - 2;
+  const int groups = (NY + kRows - 1) / kRows;
+  const int j0 = 1 + (int)(blockIdx.x % groups) * kRows, k = 1 + (int)(blockIdx.x / groups);
+  const int rows = min(kRows, NY - j0 + 1);
   const long long pl = (long long)MX * MY;
   const double dx0 = a.dx, dy0 = a.dy, ddx = 1.0 / dx0, ddy = 1.0 / dy0, ddt = 1.0 / a.dt;
   const double dz_k = a.dZ[k];
   const double dzm = __dsub_rn(a.ZC[k], a.ZC[k - 1]), dzp = __dsub_rn(a.ZC[k + 1], a.ZC[k]);
-  double acc = 0.0;
-  for (int i = 1 + threadIdx.x; i <= MX - 2; i += kThreads) {
-    const long long c = (long long)i + (long long)MX * ((long long)j + (long long)MY * k);
-    const double l0 = a.lam[c], m0 = a.m[c];
-    const long long xm = c - 1, xp = c + 1, ym = c - MX, yp = c + MX, zm = c - pl, zp = c + pl;
-    const double cxm = __dmul_rn(__dmul_rn(__dmul_rn(lam_f(a.lam[xm], l0, a.m[xm], m0), dy0), dz_k), ddx);
-    const double cxp = __dmul_rn(__dmul_rn(__dmul_rn(lam_f(a.lam[xp], l0, a.m[xp], m0), dy0), dz_k), ddx);
-    const double cym = __dmul_rn(__dmul_rn(__dmul_rn(lam_f(a.lam[ym], l0, a.m[ym], m0), dx0), dz_k), ddy);
-    const double cyp = __dmul_rn(__dmul_rn(__dmul_rn(lam_f(a.lam[yp], l0, a.m[yp], m0), dx0), dz_k), ddy);
-    const double czm = __ddiv_rn(__dmul_rn(__dmul_rn(lam_f(a.lam[zm], l0, a.m[zm], m0), dx0), dy0), dzm);
-    const double czp = __ddiv_rn(__dmul_rn(__dmul_rn(lam_f(a.lam[zp], l0, a.m[zp], m0), dx0), dy0), dzp);
-    const double vxm = __dmul_rn(__dmul_rn(__dmul_rn(a.HC[0], dy0), dz_k), __dsub_rn(1.0, a.m[xm]));
-    const double vxp = __dmul_rn(__dmul_rn(__dmul_rn(a.HC[1], dy0), dz_k), __dsub_rn(1.0, a.m[xp]));
-    const double vym = __dmul_rn(__dmul_rn(__dmul_rn(a.HC[2], dx0), dz_k), __dsub_rn(1.0, a.m[ym]));
-    const double vyp = __dmul_rn(__dmul_rn(__dmul_rn(a.HC[3], dx0), dz_k), __dsub_rn(1.0, a.m[yp]));
-    const double vzm = __dmul_rn(__dmul_rn(__dmul_rn(a.HC[4], dx0), dy0), __dsub_rn(1.0, a.m[zm]));
-    const double vzp = __dmul_rn(__dmul_rn(__dmul_rn(a.HC[5], dx0), dy0), __dsub_rn(1.0, a.m[zp]));
-    double ap = 0.0;
-    if (!a.steady)
-      ap = __dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(a.rho[c], a.cp[c]), dx0), dy0), dz_k), ddt);
-    double s = __dadd_rn(cxp, cxm);
-    s = __dadd_rn(s, cyp);
-    s = __dadd_rn(s, cym);
-    s = __dadd_rn(s, czp);
-    s = __dadd_rn(s, czm);
-    s = __dadd_rn(s, vxp);
-    s = __dadd_rn(s, vxm);
-    s = __dadd_rn(s, vyp);
-    s = __dadd_rn(s, vym);
-    s = __dadd_rn(s, vzp);
-    s = __dadd_rn(s, vzm);
-    s = __dadd_rn(s, ap);
-    const double dd = __dadd_rn(__dsub_rn(1.0, m0), __dmul_rn(s, m0));
-    const double* th = a.th;
-    double ss = __dmul_rn(cxp, th[xp]);
-    ss = __dadd_rn(ss, __dmul_rn(cxm, th[xm]));
-    ss = __dadd_rn(ss, __dmul_rn(cyp, th[yp]));
-    ss = __dadd_rn(ss, __dmul_rn(cym, th[ym]));
-    ss = __dadd_rn(ss, __dmul_rn(czp, th[zp]));
-    ss = __dadd_rn(ss, __dmul_rn(czm, th[zm]));
-    const double rs = __dmul_rn(__dsub_rn(a.b[c], __dsub_rn(ss, __dmul_rn(dd, th[c]))), m0);
-    a.r[c] = rs;
-    acc += rs * rs;
+  const double yzm = __ddiv_rn(1.0, dzm), yzp = __ddiv_rn(1.0, dzp);
+  // convective factors of the six faces; with all of them finite a face to an unmasked cell adds a zero
+  __shared__ double conv[6];
+  __shared__ double acc[kRows][kThreads];
+  if (threadIdx.x < 6) {
+    const int f = threadIdx.x;
+    conv[f] = __dmul_rn(__dmul_rn(a.HC[f], f < 2 ? dy0 : dx0), f < 4 ? dz_k : dy0);
   }
-  // fixed-order block sum, then the last block adds the row partials in row order
-  __shared__ double sm[kThreads / 32];
-  __shared__ int last;
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = acc;
+#pragma unroll
+  for (int r = 0; r < kRows; ++r) acc[r][threadIdx.x] = 0.0;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int w = 0; w < kThreads / 32; ++w) t += sm[w];
-    scratch[row] = t;
-    __threadfence();
-    unsigned* ticket = reinterpret_cast<unsigned*>(scratch + kTicket);
-    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  const bool plain = isfinite(conv[0]) && isfinite(conv[1]) && isfinite(conv[2]) && isfinite(conv[3]) &&
+                     isfinite(conv[4]) && isfinite(conv[5]);
+  const double *L = a.lam, *M = a.m, *th = a.th;
+  for (int i0 = 1; i0 <= NX; i0 += kThreads) {
+    const int i = i0 + threadIdx.x;
+    const bool on = i <= NX, first = (threadIdx.x & 31) == 0;
+    const unsigned warp_on = __ballot_sync(0xffffffffu, on);
+    if (!on) continue;
+    long long c = (long long)i + (long long)MX * ((long long)j0 + (long long)MY * k);
+    double l0 = L[c], m0 = M[c], t0 = th[c], tm = th[c - MX], mm = M[c - MX];
+    double cym = __dmul_rn(__dmul_rn(__dmul_rn(lam_f(L[c - MX], l0, mm, m0), dx0), dz_k), ddy);
+    Row n = load_row(a, c, MX, pl);
+#pragma unroll 1
+    for (int r = 0; r < rows; ++r) {
+      const Row q = n;
+      if (r + 1 < rows) n = load_row(a, c + MX, MX, pl);
+      const double cxp = __dmul_rn(__dmul_rn(__dmul_rn(lam_f(q.lxp, l0, q.mxp, m0), dy0), dz_k), ddx);
+      const double cyp = __dmul_rn(__dmul_rn(__dmul_rn(lam_f(q.lyp, l0, q.myp, m0), dx0), dz_k), ddy);
+      const double czm = div_by(__dmul_rn(__dmul_rn(lam_f(q.lzm, l0, q.mzm, m0), dx0), dy0), dzm, yzm);
+      const double czp = div_by(__dmul_rn(__dmul_rn(lam_f(q.lzp, l0, q.mzp, m0), dx0), dy0), dzp, yzp);
+      double cxm = __shfl_up_sync(warp_on, cxp, 1);
+      if (first) cxm = __dmul_rn(__dmul_rn(__dmul_rn(lam_f(L[c - 1], l0, q.mxm, m0), dy0), dz_k), ddx);
+      double s = __dadd_rn(cxp, cxm);
+      s = __dadd_rn(s, cyp);
+      s = __dadd_rn(s, cym);
+      s = __dadd_rn(s, czp);
+      s = __dadd_rn(s, czm);
+      const bool inner = plain && m0 == 1.0 && mm == 1.0 && q.mxm == 1.0 && q.mxp == 1.0 && q.myp == 1.0 &&
+                         q.mzm == 1.0 && q.mzp == 1.0;
+      if (!inner) {
+        s = __dadd_rn(s, __dmul_rn(conv[1], __dsub_rn(1.0, q.mxp)));
+        s = __dadd_rn(s, __dmul_rn(conv[0], __dsub_rn(1.0, q.mxm)));
+        s = __dadd_rn(s, __dmul_rn(conv[3], __dsub_rn(1.0, q.myp)));
+        s = __dadd_rn(s, __dmul_rn(conv[2], __dsub_rn(1.0, mm)));
+        s = __dadd_rn(s, __dmul_rn(conv[5], __dsub_rn(1.0, q.mzp)));
+        s = __dadd_rn(s, __dmul_rn(conv[4], __dsub_rn(1.0, q.mzm)));
+      }
+      double ap = 0.0;
+      if (!a.steady)
+        ap = __dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(a.rho[c], a.cp[c]), dx0), dy0), dz_k), ddt);
+      s = __dadd_rn(s, ap);
+      const double dd = __dadd_rn(__dsub_rn(1.0, m0), __dmul_rn(s, m0));
+      double ss = __dmul_rn(cxp, q.txp);
+      ss = __dadd_rn(ss, __dmul_rn(cxm, q.txm));
+      ss = __dadd_rn(ss, __dmul_rn(cyp, q.typ));
+      ss = __dadd_rn(ss, __dmul_rn(cym, tm));
+      ss = __dadd_rn(ss, __dmul_rn(czp, q.tzp));
+      ss = __dadd_rn(ss, __dmul_rn(czm, q.tzm));
+      const double rs = __dmul_rn(__dsub_rn(q.b, __dsub_rn(ss, __dmul_rn(dd, t0))), m0);
+      a.r[c] = rs;
+      acc[r][threadIdx.x] = __fma_rn(rs, rs, acc[r][threadIdx.x]);
+      // on to the next row: the cell above becomes the cell
+      tm = t0;
+      mm = m0;
+      cym = cyp;
+      t0 = q.typ;
+      l0 = q.lyp;
+      m0 = q.myp;
+      c += MX;
+    }
   }
+  // fixed-order sum of each row (row number: j fastest), then the last block adds the row partials in order
+  __shared__ double sm[kRows][kThreads / 32];
+  __shared__ int last;
+#pragma unroll
+  for (int r = 0; r < kRows; ++r) {
+    double v = acc[r][threadIdx.x];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) sm[r][threadIdx.x >> 5] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x < rows) {
+    double t = 0.0;
+    for (int w = 0; w < kThreads / 32; ++w) t += sm[threadIdx.x][w];
+    scratch[(j0 - 1 + threadIdx.x) + NY * (k - 1)] = t;
+    __threadfence();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0)
+    last = atomicInc(reinterpret_cast<unsigned*>(scratch + kTicket), gridDim.x - 1) == gridDim.x - 1;
   __syncthreads();
   if (!last) return;
   __threadfence();
   double t = 0.0;
-  for (int q = threadIdx.x; q < (int)gridDim.x; q += kThreads) t += __ldcg(scratch + q);
+  const int n = NY * NZ;
+  for (int q0 = threadIdx.x; q0 < n; q0 += 16 * kThreads) {
+    double v[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) v[u] = q0 + u * kThreads < n ? __ldcg(scratch + q0 + u * kThreads) : 0.0;
+#pragma unroll
+    for (int u = 0; u < 16; ++u) t += v[u];
+  }
   for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = t;
+  if ((threadIdx.x & 31) == 0) sm[0][threadIdx.x >> 5] = t;
   __syncthreads();
   if (threadIdx.x == 0) {
     double tot = 0.0;
-    for (int w = 0; w < kThreads / 32; ++w) tot += sm[w];
+    for (int w = 0; w < kThreads / 32; ++w) tot += sm[0][w];
     scratch[kResult] = sqrt(tot);
   }
 }
@@ -182,7 +273,8 @@ extern "C" int h2g_calcrk_noalloc(int MX, int MY, int MZ, const double* theta, c
   for (int f = 0; f < 6; ++f) a.HC[f] = HC[f];
   a.steady = is_steady ? 1 : 0;
   a.r = r;
-  k_calcrk_rows<<<(unsigned)rows, kThreads, 0, st>>>(a, scratch);
+  const unsigned blocks = (unsigned)(((MY - 2 + kRows - 1) / kRows) * (MZ - 2));
+  k_calcrk_rows<<<blocks, kThreads, 0, st>>>(a, scratch);
   if (cudaGetLastError() != cudaSuccess) return H2G_CUDA_ERROR;
   if (cudaMemcpyAsync(res, scratch + kResult, sizeof(double), cudaMemcpyDeviceToHost, st) != cudaSuccess)
     return H2G_CUDA_ERROR;
