@@ -197,7 +197,8 @@ __device__ __forceinline__ bool cell_coef(const OpParams<T>& op, int k, uint8_t 
 // pair.  k_class_coef fills one table row per class with cell_coef itself, for a steady grid, so
 // every value is the one cell_coef gives the cell; a cell then reads a 2-byte class index and one
 // 64-byte row instead of the 8-byte key word, six table entries and dd.  A transient grid adds
-// a_p0 per cell, so there dd is read from the per-cell array (the same value again).
+// a_p0 per cell: with at most kMaxKeys distinct (key, rho*cp) pairs the pair takes the own key's place in
+// the class and dd is the table's again, else dd is read from the per-cell array (the same value).
 constexpr int kClassSlots = 1 << 17;   // hash slots of the (plane, keys) pairs
 constexpr int kMaxClasses = 65535;     // class indices are 16-bit; 0xffff marks "not updated"
 
@@ -215,7 +216,7 @@ __device__ __forceinline__ bool class_coef(const OpParams<T>& op, unsigned cl, i
     c.cyp = b.y;
     c.czm = z.x;
     c.czp = z.y;
-    c.dd = op.steady ? __ldg(reinterpret_cast<const double*>(t + 3)) : __ldg(op.ddv + ci);
+    c.dd = op.cls_dd ? __ldg(reinterpret_cast<const double*>(t + 3)) : __ldg(op.ddv + ci);
   } else {
     const float4* t = reinterpret_cast<const float4*>(op.ctab) + 2 * cl;
     const float4 a = __ldg(t), z = __ldg(t + 1);
@@ -225,7 +226,7 @@ __device__ __forceinline__ bool class_coef(const OpParams<T>& op, unsigned cl, i
     c.cyp = a.w;
     c.czm = z.x;
     c.czp = z.y;
-    c.dd = op.steady ? z.z : __ldg(op.ddv + ci);
+    c.dd = op.cls_dd ? z.z : __ldg(op.ddv + ci);
   }
   return true;
 }
@@ -1357,17 +1358,21 @@ __global__ void __launch_bounds__(256) k_make_nkeys(Geo g, const uint8_t* __rest
 __device__ __forceinline__ unsigned class_hash(unsigned long long w) {
   return (unsigned)((w * 0x9E3779B97F4A7C15ull) >> (64 - 17)) & (kClassSlots - 1);
 }
-__device__ __forceinline__ unsigned long long class_word(const unsigned long long* nk, int o, int k) {
-  return (nk[o] & 0x00ffffffffffffffull) | ((unsigned long long)k << 56);
+// pair (may be null): per cell, its (key, rho*cp) pair in place of its own key.
+__device__ __forceinline__ unsigned long long class_word(const unsigned long long* nk, const uint8_t* pair, int o,
+                                                         int k) {
+  const unsigned long long w = (nk[o] & 0x00ffffffffffffffull) | ((unsigned long long)k << 56);
+  return pair ? (w & ~0xffull) | pair[o] : w;
 }
 __global__ void __launch_bounds__(256) k_class_insert(Geo g, const unsigned long long* __restrict__ nk,
+                                                       const uint8_t* __restrict__ pair,
                                                        unsigned long long* slots, int* overflow) {
   const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
   const int j = 1 + blockIdx.y, k = 1 + blockIdx.z;
   if (i > g.NX) return;
   const int o = g.off(i, j, k);
   if (!(nk[o] & 0x80)) return;  // masked: never updated
-  const unsigned long long w = class_word(nk, o, k);
+  const unsigned long long w = class_word(nk, pair, o, k);
   unsigned h = class_hash(w);
   for (int t = 0; t < kClassSlots; ++t) {
     const unsigned long long prev = atomicCAS(slots + h, 0ull, w);
@@ -1380,6 +1385,7 @@ __global__ void __launch_bounds__(256) k_class_insert(Geo g, const unsigned long
 // Step 2 (after the host numbered the occupied slots): the class index of every cell; cells that
 // are never updated (guards, masked cells, padding) keep kNoClass from the fill before.
 __global__ void __launch_bounds__(256) k_class_assign(Geo g, const unsigned long long* __restrict__ nk,
+                                                       const uint8_t* __restrict__ pair,
                                                        const unsigned long long* __restrict__ slots,
                                                        const uint16_t* __restrict__ slot_class,
                                                        uint16_t* __restrict__ cls) {
@@ -1388,7 +1394,7 @@ __global__ void __launch_bounds__(256) k_class_assign(Geo g, const unsigned long
   if (i > g.NX) return;
   const int o = g.off(i, j, k);
   if (!(nk[o] & 0x80)) return;
-  const unsigned long long w = class_word(nk, o, k);
+  const unsigned long long w = class_word(nk, pair, o, k);
   unsigned h = class_hash(w);
   for (int t = 0; t < kClassSlots; ++t) {
     const unsigned long long v = slots[h];
@@ -1403,18 +1409,27 @@ __global__ void __launch_bounds__(256) k_class_assign(Geo g, const unsigned long
 
 // Step 3: one table row per class from cell_coef on the class's (plane, keys) pair, with the
 // grid taken as steady (a_p0 = 0: dd is then the sum of the 12 face terms, what a steady cell of
-// the class gets), in the precision of the tables op points to.
+// the class gets) or, with pair_key (the key of every pair; op.rc: its rho*cp), with the pair's a_p0, in the
+// precision of the tables op points to.
 template <typename T>
 __global__ void __launch_bounds__(128) k_class_coef(OpParams<T> op, const unsigned long long* __restrict__ words,
-                                                     int ncls, T* __restrict__ ctab, int* no_recip) {
+                                                     int ncls, T* __restrict__ ctab, int* no_recip,
+                                                     const uint8_t* __restrict__ pair_key) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ncls) return;
   const unsigned long long w = words[c];
   const int k = (int)(w >> 56);
+  uint8_t own = (uint8_t)w;
+  int pair = 0;
   op.steady = 1;
+  if (pair_key) {
+    op.steady = 0;
+    pair = own & 0x7f;
+    own = pair_key[pair] | 0x80;
+  }
   Coef<T> cf;
-  cell_coef<T, false>(op, k, (uint8_t)w, (uint8_t)(w >> 8), (uint8_t)(w >> 16), (uint8_t)(w >> 24),
-                      (uint8_t)(w >> 32), (uint8_t)(w >> 40), (uint8_t)(w >> 48), 0, cf);
+  cell_coef<T, false>(op, k, own, (uint8_t)(w >> 8), (uint8_t)(w >> 16), (uint8_t)(w >> 24),
+                      (uint8_t)(w >> 32), (uint8_t)(w >> 40), (uint8_t)(w >> 48), pair, cf);
   T* t = ctab + 8 * (size_t)c;
   t[0] = cf.cxm;
   t[1] = cf.cxp;
@@ -1486,6 +1501,69 @@ __global__ void k_make_keys(Geo g, const double* __restrict__ lam, const double*
   const long long o = g.off(i, j, k);
   key[o] = (uint8_t)(idx | (mask[c] == 1.0 ? 0x80 : 0));
   if (rc) rc[o] = (T)(rho[c] * cp[c]);
+}
+
+// ------------------------------------------------------------------------------------------
+// (key, rho*cp) pairs of a transient grid's updated cells.  Pass 1 collects the distinct rho*cp bit
+// patterns like the lambda values; pass 2 marks the pairs key | index << 7 that occur; pass 3 writes
+// each cell's pair number | 0x80 (numbered by the host; 0 where the cell is never updated).
+// ------------------------------------------------------------------------------------------
+__device__ __forceinline__ int slot_of(const unsigned long long* slots, unsigned long long b) {
+  unsigned h = slot_hash(b);
+  for (int probe = 0; probe < kHashSlots; ++probe, h = (h + 1) & (kHashSlots - 1))
+    if (slots[h] == b) return (int)h;
+  return 0;
+}
+
+__global__ void __launch_bounds__(256) k_collect_rc(Geo g, const uint8_t* __restrict__ key,
+                                                     const double* __restrict__ rc, unsigned long long* slots,
+                                                     int* flags) {
+  const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = 1 + blockIdx.y, k = 1 + blockIdx.z;
+  if (i > g.NX || *flags) return;  // too many already: the pairs are given up
+  const int o = g.off(i, j, k);
+  if (!(key[o] & 0x80)) return;
+  const unsigned long long b = (unsigned long long)__double_as_longlong(rc[o]);
+  unsigned h = slot_hash(b);
+  for (int probe = 0; probe < kHashSlots; ++probe, h = (h + 1) & (kHashSlots - 1)) {
+    unsigned long long cur = slots[h];
+    if (cur == b) return;
+    if (cur == ~0ull) {
+      cur = atomicCAS(slots + h, ~0ull, b);
+      if (cur == ~0ull || cur == b) return;
+    }
+  }
+  atomicOr(flags, kFlagTooMany);
+}
+
+__global__ void __launch_bounds__(256) k_mark_pairs(Geo g, const uint8_t* __restrict__ key,
+                                                     const double* __restrict__ rc,
+                                                     const unsigned long long* __restrict__ slots,
+                                                     const int* __restrict__ slot_index, unsigned* bits) {
+  const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = 1 + blockIdx.y, k = 1 + blockIdx.z;
+  if (i > g.NX) return;
+  const int o = g.off(i, j, k);
+  if (!(key[o] & 0x80)) return;
+  const int id = (key[o] & 0x7f) | slot_index[slot_of(slots, (unsigned long long)__double_as_longlong(rc[o]))] << 7;
+  if (!(bits[id >> 5] >> (id & 31) & 1u)) atomicOr(bits + (id >> 5), 1u << (id & 31));
+}
+
+__global__ void __launch_bounds__(256) k_write_pairs(Geo g, const uint8_t* __restrict__ key,
+                                                      const double* __restrict__ rc,
+                                                      const unsigned long long* __restrict__ slots,
+                                                      const int* __restrict__ slot_index,
+                                                      const uint8_t* __restrict__ number, uint8_t* __restrict__ pair) {
+  const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = 1 + blockIdx.y, k = 1 + blockIdx.z;
+  if (i > g.NX) return;
+  const int o = g.off(i, j, k);
+  if (!(key[o] & 0x80)) {
+    pair[o] = 0;
+    return;
+  }
+  const int id = (key[o] & 0x7f) | slot_index[slot_of(slots, (unsigned long long)__double_as_longlong(rc[o]))] << 7;
+  pair[o] = number[id] | 0x80;
 }
 
 }  // namespace h2g

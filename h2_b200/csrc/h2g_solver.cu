@@ -189,6 +189,13 @@ struct Solver {
   uint16_t* slot_class = nullptr;
   unsigned long long* cwords = nullptr;
   int* cflag = nullptr;
+  // transient grids: (key, rho*cp) pairs in the classes (cls_rc), per cell and their keys and rho*cp
+  bool cls_rc = false;
+  uint8_t* pair = nullptr;
+  uint8_t* pair_num = nullptr;  // 2^15 pair numbers, then the pairs' keys (128)
+  unsigned* pair_bits = nullptr;
+  double* pair_rc64 = nullptr;
+  float* pair_rc32 = nullptr;
   bool rb_tuned = false;  // rb_rows chosen (by the tuner or h2g_set_tuning)
   // fused sweeps (k_rb_sweep): sweeps 2-5 of the preconditioner as one launch each, ping-ponging
   // between the preconditioner's output and x2 (one per precision; guards zero, never written)
@@ -559,7 +566,7 @@ class SmLease {
 static ResidentPlan resident_plan(const Solver* s) {
   ResidentPlan no, pl;
   const Geo& g = s->g;
-  if (s->precision != H2G_FP64 || !s->cls_ok || !s->recip_ok || !s->steady || s->nrhs) return no;
+  if (s->precision != H2G_FP64 || !s->cls_ok || !s->recip_ok || !(s->steady || s->cls_rc) || s->nrhs) return no;
   if (s->tuning_forced || s->sweep_forced >= 0 || s->coop_forced >= 0 || s->device >= kMaxDevices) return no;
   for (const char* e : {"H2G_RB_ROWS", "H2G_RB_PLANES", "H2G_RB_DD", "H2G_AX_DD", "H2G_RB_FUSED", "H2G_SW_CHUNKS",
                         "H2G_SW_DD", "H2G_RB_COOP"})
@@ -765,6 +772,7 @@ static OpParams<T> op_params_rc(const Solver* s, const OpTables<T>& t, const T* 
   op.nkey = s->nkey;
   op.cls = nullptr;
   op.ctab = nullptr;
+  op.cls_dd = s->steady || s->cls_rc;
   const double dx0 = s->dx, dy0 = s->dy;
   op.czm = (T)((s->HC[4] * dx0) * dy0);
   op.czp = (T)((s->HC[5] * dx0) * dy0);
@@ -826,6 +834,7 @@ static void destroy(Solver* s) {
   for (auto& p : s->stage) cudaFree(p);
   cudaFree(s->x2_64); cudaFree(s->x2_32); cudaFree(s->sweep_err); cudaFree(s->gbar);
   cudaFree(s->cls); cudaFree(s->ctab); cudaFree(s->ctab32); cudaFree(s->cslots); cudaFree(s->slot_class); cudaFree(s->cwords);
+  cudaFree(s->pair); cudaFree(s->pair_num); cudaFree(s->pair_bits); cudaFree(s->pair_rc64); cudaFree(s->pair_rc32);
   cudaFree(s->cflag); cudaFree(s->key_prev); cudaFree(s->kdiff);
   cudaFree(s->rs_box); cudaFree(s->rs_rowsum); cudaFree(s->rs_ctl); cudaFree(s->rs_lcls); cudaFree(s->rs_list);
   cudaFree(s->rs_count);
@@ -882,12 +891,77 @@ static void invalidate_graphs(Solver* s) {
 // and their coefficients.  Left unbuilt (the kernels keep the key tables) when disabled
 // (H2G_CLS=0), when NZ > 255 (the plane shares the 64-bit word with the keys) or when the grid has
 // more than kMaxClasses pairs.
+// The (key, rho*cp) pairs of a transient grid: s->pair per cell and the pairs' keys and rho*cp on the
+// device.  *ok = false (and the classes then hold no a_p0) with more than 256 values of rho*cp or more than
+// kMaxKeys pairs.
+static int build_pairs(Solver* s, bool* ok) {
+  const Geo& g = s->g;
+  *ok = false;
+  constexpr int kIds = 1 << 15;
+  if (!s->pair) {
+    CK(cudaMalloc(&s->pair, (size_t)g.n));
+    CK(cudaMalloc(&s->pair_num, kIds + 128));
+    CK(cudaMalloc(&s->pair_bits, kIds / 8));
+    CK(cudaMalloc(&s->pair_rc64, sizeof(double) * 128));
+    CK(cudaMalloc(&s->pair_rc32, sizeof(float) * 128));
+  }
+  const dim3 gi((g.NX + 255) / 256, g.NY, g.NZ);
+  CK(cudaMemsetAsync(s->slots, 0xff, sizeof(unsigned long long) * kHashSlots, s->stream));
+  CK(cudaMemsetAsync(s->flags, 0, sizeof(int), s->stream));
+  CK(cudaMemsetAsync(s->pair_bits, 0, kIds / 8, s->stream));
+  k_collect_rc<<<gi, 256, 0, s->stream>>>(g, s->key, s->rc64, s->slots, s->flags);
+  CKL();
+  std::vector<unsigned long long> slots(kHashSlots);
+  int flags = 0;
+  CK(cudaMemcpyAsync(slots.data(), s->slots, sizeof(unsigned long long) * kHashSlots, cudaMemcpyDeviceToHost, s->stream));
+  CK(cudaMemcpyAsync(&flags, s->flags, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+  CK(cudaStreamSynchronize(s->stream));
+  if (flags) return H2G_OK;
+  std::vector<int> index(kHashSlots, 0);
+  std::vector<double> value;
+  for (int h = 0; h < kHashSlots; ++h)
+    if (slots[h] != ~0ull) {
+      index[h] = (int)value.size();
+      double v;
+      memcpy(&v, &slots[h], sizeof v);
+      value.push_back(v);
+    }
+  CK(cudaMemcpyAsync(s->slot_index, index.data(), sizeof(int) * kHashSlots, cudaMemcpyHostToDevice, s->stream));
+  k_mark_pairs<<<gi, 256, 0, s->stream>>>(g, s->key, s->rc64, s->slots, s->slot_index, s->pair_bits);
+  CKL();
+  std::vector<unsigned> bits(kIds / 32);
+  CK(cudaMemcpyAsync(bits.data(), s->pair_bits, kIds / 8, cudaMemcpyDeviceToHost, s->stream));
+  CK(cudaStreamSynchronize(s->stream));
+  std::vector<uint8_t> num(kIds + 128, 0);
+  std::vector<double> rc64(128, 0.0);
+  std::vector<float> rc32(128, 0.0f);
+  int n = 0;
+  for (int id = 0; id < kIds; ++id) {
+    if (!(bits[id >> 5] >> (id & 31) & 1u)) continue;
+    if (n >= kMaxKeys) return H2G_OK;
+    num[id] = (uint8_t)n;
+    num[kIds + n] = (uint8_t)(id & 0x7f);
+    rc64[n] = value[id >> 7];
+    rc32[n] = (float)value[id >> 7];
+    ++n;
+  }
+  CK(cudaMemcpyAsync(s->pair_num, num.data(), num.size(), cudaMemcpyHostToDevice, s->stream));
+  CK(cudaMemcpyAsync(s->pair_rc64, rc64.data(), sizeof(double) * 128, cudaMemcpyHostToDevice, s->stream));
+  CK(cudaMemcpyAsync(s->pair_rc32, rc32.data(), sizeof(float) * 128, cudaMemcpyHostToDevice, s->stream));
+  k_write_pairs<<<gi, 256, 0, s->stream>>>(g, s->key, s->rc64, s->slots, s->slot_index, s->pair_num, s->pair);
+  CKL();
+  CK(cudaStreamSynchronize(s->stream));  // the host vectors must outlive the copies
+  *ok = n > 0;
+  return H2G_OK;
+}
+
 static int build_classes(Solver* s) {
   const Geo& g = s->g;
   const bool was = s->cls_ok;
   s->cls_ok = false;
   s->ncls = 0;
   s->rs_ntab = 0;
+  s->cls_rc = false;
   const char* e = getenv("H2G_CLS");
   if ((e && atoi(e) == 0) || g.NZ > 255 || !s->nkey) {
     if (was) invalidate_graphs(s);
@@ -902,11 +976,16 @@ static int build_classes(Solver* s) {
     CK(cudaMalloc(&s->cwords, sizeof(unsigned long long) * kMaxClasses));
     CK(cudaMalloc(&s->cflag, sizeof(int)));
   }
+  bool pairs = false;
+  if (!s->steady && s->rc64)
+    if (int rc = build_pairs(s, &pairs)) return rc;
+  const uint8_t* pair = pairs ? s->pair : nullptr;
+  const uint8_t* pair_key = pairs ? s->pair_num + (1 << 15) : nullptr;
   CK(cudaMemsetAsync(s->cslots, 0, sizeof(unsigned long long) * kClassSlots, s->stream));
   CK(cudaMemsetAsync(s->cflag, 0, sizeof(int), s->stream));
   CK(cudaMemsetAsync(s->cls, 0xff, sizeof(uint16_t) * (size_t)g.n, s->stream));
   const dim3 gi((g.NX + 255) / 256, g.NY, g.NZ);
-  k_class_insert<<<gi, 256, 0, s->stream>>>(g, s->nkey, s->cslots, s->cflag);
+  k_class_insert<<<gi, 256, 0, s->stream>>>(g, s->nkey, pair, s->cslots, s->cflag);
   CKL();
   std::vector<unsigned long long> slots(kClassSlots);
   int flag = 0;
@@ -932,20 +1011,21 @@ static int build_classes(Solver* s) {
   CK(cudaMemcpyAsync(s->slot_class, sc.data(), sizeof(uint16_t) * kClassSlots, cudaMemcpyHostToDevice, s->stream));
   CK(cudaMemcpyAsync(s->cwords, words.data(), sizeof(unsigned long long) * words.size(), cudaMemcpyHostToDevice,
                      s->stream));
-  k_class_assign<<<gi, 256, 0, s->stream>>>(g, s->nkey, s->cslots, s->slot_class, s->cls);
+  k_class_assign<<<gi, 256, 0, s->stream>>>(g, s->nkey, pair, s->cslots, s->slot_class, s->cls);
   const int ncls = (int)words.size();
-  OpParams<double> o64 = op_params_rc<double>(s, s->t64, s->rc64);
+  OpParams<double> o64 = op_params_rc<double>(s, s->t64, pairs ? s->pair_rc64 : s->rc64);
   CK(cudaMemsetAsync(s->cflag, 0, sizeof(int), s->stream));
-  k_class_coef<double><<<(ncls + 127) / 128, 128, 0, s->stream>>>(o64, s->cwords, ncls, s->ctab, s->cflag);
+  k_class_coef<double><<<(ncls + 127) / 128, 128, 0, s->stream>>>(o64, s->cwords, ncls, s->ctab, s->cflag, pair_key);
   if (s->ctab32) {
-    OpParams<float> o32 = op_params_rc<float>(s, s->t32, s->rc32);
-    k_class_coef<float><<<(ncls + 127) / 128, 128, 0, s->stream>>>(o32, s->cwords, ncls, s->ctab32, nullptr);
+    OpParams<float> o32 = op_params_rc<float>(s, s->t32, pairs ? s->pair_rc32 : s->rc32);
+    k_class_coef<float><<<(ncls + 127) / 128, 128, 0, s->stream>>>(o32, s->cwords, ncls, s->ctab32, nullptr, pair_key);
   }
   CKL();
   CK(cudaMemcpyAsync(&flag, s->cflag, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));  // the host vectors must outlive the copies
   s->ncls = ncls;
   s->recip_ok = flag == 0;
+  s->cls_rc = pairs;
   s->cls_ok = true;
   if (!was) invalidate_graphs(s);
   return H2G_OK;

@@ -62,6 +62,31 @@ def test_preconditioner_masked_cells(oracle):
     s.close()
 
 
+@pytest.mark.parametrize("n", [(41, 37, 30), (121, 70, 30), (198, 181, 30)], ids=lambda n: "x".join(map(str, n)))
+def test_transient_grid(oracle, n):
+    """a_p0 in the class table: the preconditioner gives the oracle's bits, a solve those of the colour passes,
+    and a grid with more (key, rho cp) pairs than a class holds keeps the colour passes."""
+    prob = mode3_model(oracle, n[0], n[1], n[2], is_steady=False, dt=1e-4)
+    s = make_solver(prob)
+    bb = random_interior(prob.shape, 8)
+    assert np.array_equal(s.preconditioner(bb, "gs"), oracle.preconditioner(prob, bb, "gs"))
+    s.snapshot()
+    st, res = s.solve("pbicgstab", tol=1e-8, maxItr=100, smoother="gs")
+    th = s.get_theta()
+    assert res.launches == launches_of(s, res.itr)
+    s.snapshot(restore=True)
+    s.set_tuning(8, 2)
+    assert s.solve("pbicgstab", tol=1e-8, maxItr=100, smoother="gs")[1].itr == res.itr
+    assert np.array_equal(s.get_theta(), th)
+    s.set_tuning(0)
+    prob.wk["rho"][1:-1, 1:-1, 1:-1] *= 1.0 + 0.01 * np.random.default_rng(3).integers(0, 40, (n[0], n[1], n[2]))
+    s.set_fields(prob.wk["lam"], prob.wk["mask"], prob.wk["rho"], prob.wk["cp"])
+    assert np.array_equal(s.preconditioner(bb, "gs"), oracle.preconditioner(prob, bb, "gs"))
+    st, res = s.solve("pbicgstab", tol=1e-8, maxItr=100, smoother="gs")
+    assert res.launches != launches_of(s, res.itr)
+    s.close()
+
+
 @pytest.mark.parametrize("method", ["pbicgstab", "cg"])
 @pytest.mark.parametrize("n", [(24, 20, 30), (41, 37, 30), (121, 117, 30), (200, 230, 30), (66, 50, 60)],
                          ids=lambda n: "x".join(map(str, n)))
