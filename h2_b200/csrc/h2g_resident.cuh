@@ -38,7 +38,7 @@ namespace h2g {
 
 constexpr int kRsRowPitch = 34;   // doubles per row in shared memory: 32 positions and one on each side
 constexpr int kRsBox = 72;        // messages per tile, plane and colour: first row, last row, x edges
-constexpr int kRsZero = 4 * kRsBox;  // slots behind the last tile's that nobody writes (zeros)
+constexpr int kRsZero = 4 * kRsBox;  // slots before the first tile's that nobody writes (zeros)
 constexpr int kRsMaxRows = 8;
 constexpr int kRsMaxWarps = 15;   // 136 registers a thread
 
@@ -553,7 +553,7 @@ __global__ void __launch_bounds__(32 * kRsMaxWarps, 1) k_resident(const __grid_c
   // where the messages, rows and classes of the pair of planes pl0, pl0 + 1 are
   auto pair_at = [&](int pl0) {
     RsPair a;
-    const ulonglong2* zero = A.box + (size_t)gridDim.x * NZe * (2 * kRsBox);
+    const ulonglong2* zero = A.box - kRsZero;
     a.box = box_of(tile, pl0) + lane;
     a.mlo = n_lo ? ~0u : 0u;
     a.mhi = n_hi ? ~0u : 0u;

@@ -161,7 +161,7 @@ struct Solver {
   size_t partials_cap = 0;
   double* hist = nullptr;
   int hist_cap = 0;
-  SolveGraph graphs[kGNum][3];  // smoother none, gs, gs with the resident preconditioner
+  SolveGraph graphs[kGNum][4];  // smoother none, gs, gs with the resident preconditioner on all SMs, on a share
   // mixed-precision refinement settings
   double inner_tol = 1e-4;
   int max_outer = 40;
@@ -212,6 +212,7 @@ struct Solver {
   double div_limit = 0.0;   // divergence stop of the next solves' states (mixed FP32 passes only)
   int coop_blocks = 0;      // blocks of the launch: SMs x resident blocks per SM
   bool coop_barred = false; // set while h2g_batch_solve runs the handle beside others
+  int sm_share = 0;         // SMs k_resident may take there (0: all)
   GridBar* gbar = nullptr;
   long long wait_limit = kWaitCycles;  // budget of one bounded wait (clock cycles)
   std::map<std::pair<const void*, int>, CUtensorMap> xmaps;  // TMA maps of x buffers (pointer, bytes/element)
@@ -227,6 +228,7 @@ struct Solver {
   uint16_t* rs_list = nullptr;
   int* rs_count = nullptr;
   int rs_ntab = 0;              // rows of the largest tile table (0: to be made)
+  int rs_rows = 0;              // R of the split that the tables are for
   size_t rs_smem = 0;
   bool rs_fits = false;
   // K right-hand sides on the handle's operator (h2g_create_multi): stacked vectors, K states
@@ -558,7 +560,10 @@ class SmLease {
 };
 
 // The split of k_resident for a grid, if it has one: tiles of 32 positions x R rows x all planes with
-// the fewest rows (the shortest pass) for which there is an SM for every tile.  A warp has one pair of
+// the fewest rows (the shortest pass) for which there is an SM for every tile; in a batch, first within
+// the handle's share of them.  A pass grows more slowly than its rows (its messages and barriers stay), so
+// two solves on halves beat two in turn on all: 120^2, 180^2 and 240^2 twice each, two threads, in turn 224 ms,
+// the first two on halves 192 ms (colour passes beside each other 218 ms).  A warp has one pair of
 // planes up to 30 planes (up to 8 rows: 240x240x30 takes 7, 140 tiles), two pairs up to 60 planes (4
 // rows).  Larger grids keep the separate launches, as do the grids without a class table or with tiles of
 // too many classes (resident_prepare), the FP32 smoother, and handles on which a launch shape, a
@@ -574,10 +579,11 @@ static ResidentPlan resident_plan(const Solver* s) {
   pl.np = g.NZ <= 2 * kRsMaxWarps ? 1 : 2;
   if (g.NZ > 4 * kRsMaxWarps) return no;
   pl.nxb = (g.HN + 31) / 32;
-  for (pl.R = 1; pl.R <= (pl.np == 1 ? kRsMaxRows : 4); ++pl.R) {
-    pl.ntj = (g.NY + pl.R - 1) / pl.R;
-    if (pl.blocks() <= s->num_sms) return pl;
-  }
+  for (int sms : {s->sm_share, s->num_sms})
+    for (pl.R = 1; pl.R <= (pl.np == 1 ? kRsMaxRows : 4); ++pl.R) {
+      pl.ntj = (g.NY + pl.R - 1) / pl.R;
+      if (pl.blocks() <= sms) return pl;
+    }
   return no;
 }
 
@@ -585,7 +591,8 @@ static ResidentPlan resident_plan(const Solver* s) {
 // return: a tile has more classes than fit beside its x and b.
 static int resident_prepare(Solver* s, ResidentPlan& pl) {
   const Geo& g = s->g;
-  const size_t box = sizeof(ulonglong2) * ((size_t)pl.blocks() * ((g.NZ + 1) & ~1) * 2 * kRsBox + kRsZero);
+  // room for every split: a handle may run with all SMs in one call and a share of them in the next
+  const size_t box = sizeof(ulonglong2) * ((size_t)s->num_sms * ((g.NZ + 1) & ~1) * 2 * kRsBox + kRsZero);
   if (!s->rs_ctl) {
     const size_t nb = (size_t)pl.nxb * ((g.NY + kBY - 1) / kBY) * g.NZ;
     CK(cudaMalloc(&s->rs_box, box));
@@ -596,8 +603,8 @@ static int resident_prepare(Solver* s, ResidentPlan& pl) {
     CK(cudaMemset(s->rs_rowsum, 0, s->rs_rowsum_cap));
     CK(cudaMalloc(&s->rs_lcls, sizeof(uint16_t) * (size_t)g.n));
     CK(cudaMemset(s->rs_lcls, 0, sizeof(uint16_t) * (size_t)g.n));
-    CK(cudaMalloc(&s->rs_list, sizeof(uint16_t) * (size_t)pl.blocks() * kRsMaxTab));
-    CK(cudaMalloc(&s->rs_count, sizeof(int) * (size_t)pl.blocks()));
+    CK(cudaMalloc(&s->rs_list, sizeof(uint16_t) * (size_t)s->num_sms * kRsMaxTab));
+    CK(cudaMalloc(&s->rs_count, sizeof(int) * (size_t)s->num_sms));
     RsCtl* c = nullptr;
     CK(cudaMalloc(&c, sizeof(RsCtl)));
     const RsCtl init{1ull, 0u, 0u};
@@ -608,7 +615,9 @@ static int resident_prepare(Solver* s, ResidentPlan& pl) {
     s->rs_ctl = c;
     s->rs_ntab = 0;
   }
-  if (!s->rs_ntab) {  // the classes were built anew
+  if (!s->rs_ntab || s->rs_rows != pl.R) {  // the classes were built anew, or another split
+    s->rs_ntab = 0;
+    s->rs_rows = pl.R;
     std::vector<int> count(pl.blocks());
     CK(launch_tile_classes(s->stream, g, s->cls, s->rs_lcls, s->rs_list, s->rs_count, pl.R, pl.nxb, pl.ntj));
     CK(cudaMemcpyAsync(count.data(), s->rs_count, sizeof(int) * count.size(), cudaMemcpyDeviceToHost, s->stream));
@@ -641,7 +650,7 @@ static int launch_resident(Solver* s, cudaStream_t cs, const OpParams<double>& o
   a.st = st;
   a.rowsum = s->rs_rowsum;
   a.partials = s->partials;
-  a.box = s->rs_box;
+  a.box = s->rs_box + kRsZero;
   a.ctl = s->rs_ctl;
   a.lcls = s->rs_lcls;
   a.list = s->rs_list;
@@ -1325,7 +1334,7 @@ template <typename T, typename TX, typename TP>
 static int get_graph(Solver* s, int kind, int smoother, const OpParams<T>& op, const OpParams<TP>& opM, TX* x,
                      SolverState* st, SolveGraph** out) {
   const bool resident = std::is_same<T, double>::value && std::is_same<TP, double>::value && s->rs.R && smoother;
-  SolveGraph& G = s->graphs[kind][resident ? 2 : smoother ? 1 : 0];
+  SolveGraph& G = s->graphs[kind][resident ? (s->sm_share ? 3 : 2) : smoother ? 1 : 0];
   std::vector<unsigned char> sig = signature(op, opM, smoother, (const void*)x);
   sig.push_back(use_coop(s) ? 1 : 0);
   if (resident) {
@@ -3101,11 +3110,28 @@ int h2g_batch_solve(int n, h2g_solver* const* hs, int method, double tol, int ma
   const int nt = std::max(1, std::min(threads > 0 ? threads : 2, n));
   // a cooperative launch needs the whole device: handles that run beside others use the colour
   // passes
-  for (int q = 0; q < n; ++q) S(hs[q])->coop_barred = nt > 1;
+  for (int q = 0; q < n; ++q) {
+    S(hs[q])->coop_barred = nt > 1;
+    S(hs[q])->sm_share = nt > 1 ? S(hs[q])->num_sms / nt : 0;
+  }
+  // members whose resident solve takes more than a share run one at a time: first, so that no share waits
+  // beside them; then the ones with a share, the longest first; then the others in the order given
+  std::vector<int> order(n), rank(n, 2);
+  for (int q = 0; q < n; ++q) {
+    const Solver* s = S(hs[q]);
+    order[q] = q;
+    const h2g::ResidentPlan pl = method != 2 && smoother == H2G_SMOOTHER_GS ? h2g::resident_plan(s) : h2g::ResidentPlan();
+    if (pl.R && nt > 1) rank[q] = pl.blocks() > s->sm_share ? 0 : 1;
+  }
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+    if (rank[a] != rank[b]) return rank[a] < rank[b];
+    return rank[a] == 1 && S(hs[a])->g.n > S(hs[b])->g.n;
+  });
   std::atomic<int> next(0);
   std::vector<std::string> errs(n);
   auto work = [&]() {
-    for (int q = next.fetch_add(1); q < n; q = next.fetch_add(1)) {
+    for (int i = next.fetch_add(1); i < n; i = next.fetch_add(1)) {
+      const int q = order[i];
       Solver* s = S(hs[q]);
       cudaSetDevice(s->device);
       h2g_result r{};
@@ -3127,6 +3153,7 @@ int h2g_batch_solve(int n, h2g_solver* const* hs, int method, double tol, int ma
     cudaStreamSynchronize(own[q]);
     s->stream = saved[q];
     s->coop_barred = false;
+    s->sm_share = 0;
     cudaStreamDestroy(own[q]);
   }
   int worst = H2G_OK;

@@ -162,3 +162,31 @@ def test_two_threads(oracle):
     for g in got:
         assert g[0] == 0 and g[1:3] == (rr.itr, rr.res)
         assert np.array_equal(g[3], th)
+
+
+@pytest.mark.parametrize("threads", [2, 3])
+def test_batch_shares(oracle, threads):
+    """h2g_batch_solve: members on a share of the SMs beside each other, members that need them all, and one
+    without a split; the handles alternate between a share and all SMs.  Always the lone solve's bits."""
+    sizes = [(62, 63, 30), (200, 222, 30), (62, 63, 30), (121, 117, 30), (260, 40, 30), (41, 37, 30)]
+    hs = [make_solver(mode3_model(oracle, *n)) for n in sizes]
+    for s in hs:
+        s.snapshot()
+    ptr = (ctypes.c_void_p * len(hs))(*[s.h.value for s in hs])
+    lone = None
+    for _ in range(2):
+        got = []
+        for s in hs:
+            s.snapshot(restore=True)
+            st, res = s.solve("pbicgstab", tol=1e-8, maxItr=60, smoother="gs")
+            got.append((res.itr, res.res, s.get_theta()))
+            s.snapshot(restore=True)
+        lone = lone or got
+        outs = (L.Result * len(hs))()
+        L.load().h2g_batch_solve(len(hs), ptr, 0, 1e-8, 60, 1, threads, outs)
+        got += [(o.itr, o.res, s.get_theta()) for o, s in zip(outs, hs)]
+        for q, g in enumerate(got):
+            ref = lone[q % len(hs)]
+            assert g[:2] == ref[:2] and np.array_equal(g[2], ref[2])
+    for s in hs:
+        s.close()
