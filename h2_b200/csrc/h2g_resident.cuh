@@ -101,28 +101,6 @@ __device__ __forceinline__ void msg_load(const ulonglong2* p, double& v, unsigne
   seq = (unsigned)q;
 }
 
-// a/d correctly rounded from y = RN(1/d), by two of Markstein's correction steps (P. Markstein,
-// "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34,
-// 1990): q + (a - d q) y with a fused remainder.  The first step makes q one of the two neighbours of
-// a/d, the second rounds it correctly.  The remainder is formed negated, so that a zero keeps its
-// sign.  Valid while neither the remainder nor the quotient leaves the normal range: d within
-// 2^+-100 (checked when the class table is made) and a within 2^+-400 or zero; anything else takes the
-// division (div_fix).  5 operations instead of about 39.
-__device__ __forceinline__ double div_by(double a, double d, double y) {
-  double q = __dmul_rn(a, y);
-  double r = __fma_rn(d, q, -a);
-  q = __fma_rn(-r, y, q);
-  r = __fma_rn(d, q, -a);
-  q = __fma_rn(-r, y, q);
-  return q;
-}
-// Whether a is outside that range: its exponent is, and it is not zero (the residual far from a heat source,
-// the lanes beyond the grid: a branch taken for those would be taken all the time).
-__device__ __forceinline__ bool div_bad(double a) {
-  const unsigned hi = (unsigned)__double2hiint(a), lo = (unsigned)__double2loint(a);
-  return 2u * hi - 2u * ((1023u - 400u) << 20) > 2u * (800u << 20) && ((hi & 0x7fffffffu) | lo) != 0u;
-}
-
 // Shared memory by 32-bit address and constant distance (bytes).  The compiler takes these for opaque
 // operations in program order; __syncwarp() separates them from other accesses.
 __device__ __forceinline__ unsigned saddr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }

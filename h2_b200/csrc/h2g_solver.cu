@@ -1928,18 +1928,19 @@ static int solve(Solver* s, bool cg, double tol, int maxItr, int smoother, int v
 // creation and set-up
 // ------------------------------------------------------------------------------------------
 // One rbsor! (colour 0, colour 1, each with its residual sum) with the coefficients from the key
-// tables (DDM 1) or the stencil-class table (DDM 2).
-template <int DDM>
+// tables (DDM 1) or the stencil-class table (DDM 2; RCP: its dd and omega have reciprocals for div_by).
+template <int DDM, bool RCP>
 static void sor_passes(Solver* s, cudaStream_t cs, const OpParams<double>& op, dim3 rg, dim3 blk, double omega,
                        SolverState* st, cudaGraphConditionalHandle hc, int use_cond) {
-  launch(s, k_sor_pass<false, DDM>, rg, blk, cs, op, s->th, (const double*)s->b, 0, omega, st, s->partials,
-         (int)kStageSorHalf, hc, 0);
+  const double romega = 1.0 / omega;
+  launch(s, k_sor_pass<false, DDM, 0, RCP>, rg, blk, cs, op, s->th, (const double*)s->b, omega, romega, st, s->partials,
+         hc, 0);
   if (use_cond)
-    launch(s, k_sor_pass<true, DDM>, rg, blk, cs, op, s->th, (const double*)s->b, 1, omega, st, s->partials,
-           (int)kStageSorIter, hc, use_cond);
+    launch(s, k_sor_pass<true, DDM, 1, RCP>, rg, blk, cs, op, s->th, (const double*)s->b, omega, romega, st, s->partials,
+           hc, use_cond);
   else
-    launch(s, k_sor_pass<false, DDM>, rg, blk, cs, op, s->th, (const double*)s->b, 1, omega, st, s->partials,
-           (int)kStageSorIter, hc, use_cond);
+    launch(s, k_sor_pass<false, DDM, 1, RCP>, rg, blk, cs, op, s->th, (const double*)s->b, omega, romega, st,
+           s->partials, hc, use_cond);
 }
 
 // solveSOR! (NonUniform.jl:1004-1051): res0 = resSOR, then rbsor! passes (colour 0, colour 1,
@@ -1965,10 +1966,14 @@ static int solve_sor(Solver* s, double omega, double tol, int maxItr, int verbos
   std::vector<unsigned char> sig(sizeof op + sizeof omega);
   memcpy(sig.data(), &op, sizeof op);
   memcpy(sig.data() + sizeof op, &omega, sizeof omega);
+  sig.push_back(s->recip_ok ? 1 : 0);
   if (!G.exec || G.sig != sig) {
     rc = make_loop_graph(s, G, [&](cudaStream_t cs, cudaGraphConditionalHandle hc, int use_cond) {
-      if (op.cls) sor_passes<2>(s, cs, op, rg, blk, omega, st, hc, use_cond);
-      else sor_passes<1>(s, cs, op, rg, blk, omega, st, hc, use_cond);
+      // the quotients by reciprocals need dd and omega within 2^+-100 (div_by)
+      if (op.cls && op.cls_dd && s->recip_ok && omega >= 0x1p-100)
+        sor_passes<2, true>(s, cs, op, rg, blk, omega, st, hc, use_cond);
+      else if (op.cls) sor_passes<2, false>(s, cs, op, rg, blk, omega, st, hc, use_cond);
+      else sor_passes<1, false>(s, cs, op, rg, blk, omega, st, hc, use_cond);
     });
     if (rc) return rc;
     G.sig = sig;
