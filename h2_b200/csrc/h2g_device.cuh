@@ -29,6 +29,10 @@ __device__ __forceinline__ int ld_relaxed_s32(const int* p) {
   return v;
 }
 
+__device__ __forceinline__ void set_cond(cudaGraphConditionalHandle h, int use_cond, int value) {
+  if (use_cond) cudaGraphSetConditional(h, value ? 1u : 0u);
+}
+
 // Scalar logic of each stage (runs on one thread).  Mirrors the control flow of PBiCGSTAB!
 // (NonUniform.jl:262-349) and CG! (NonUniform.jl:131-225).
 static __device__ void finish_stage(int stage, SolverState* st, double s1, double s2) {

@@ -83,10 +83,6 @@ __device__ __forceinline__ void pdl_enter() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-__device__ __forceinline__ void set_cond(cudaGraphConditionalHandle h, int use_cond, int value) {
-  if (use_cond) cudaGraphSetConditional(h, value ? 1u : 0u);
-}
-
 // A thread's share of the fixed-order sum of the blocks' partials; eight independent loads in flight.
 template <int NV>
 __device__ __forceinline__ void ordered_sum(double (&acc)[NV], const double* __restrict__ partials, unsigned nb, int tid,

@@ -39,6 +39,29 @@ const void* resident_kernel(int R, int np, int vm) {
   }
 }
 
+const void* resident_sor_kernel(int R, int np) {
+  if (np == 1) {
+    switch (R) {
+      case 1: return (const void*)k_resident_sor<1, 1, true>;
+      case 2: return (const void*)k_resident_sor<2, 1, true>;
+      case 3: return (const void*)k_resident_sor<3, 1, true>;
+      case 4: return (const void*)k_resident_sor<4, 1, true>;
+      case 5: return (const void*)k_resident_sor<5, 1, true>;
+      case 6: return (const void*)k_resident_sor<6, 1, false>;
+      case 7: return (const void*)k_resident_sor<7, 1, false>;
+      case 8: return (const void*)k_resident_sor<8, 1, false>;
+      default: return nullptr;
+    }
+  }
+  switch (R) {
+    case 1: return (const void*)k_resident_sor<1, 2, true>;
+    case 2: return (const void*)k_resident_sor<2, 2, true>;
+    case 3: return (const void*)k_resident_sor<3, 2, false>;
+    case 4: return (const void*)k_resident_sor<4, 2, false>;
+    default: return nullptr;
+  }
+}
+
 cudaError_t launch_tile_classes(cudaStream_t st, const Geo& g, const uint16_t* cls, uint16_t* lcls, uint16_t* list,
                                 int* count, int R, int nxb, int ntj) {
   k_tile_classes<<<nxb * ntj, 256, 0, st>>>(g, cls, lcls, list, count, R, nxb);

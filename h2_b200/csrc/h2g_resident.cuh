@@ -42,11 +42,11 @@ constexpr int kRsZero = 4 * kRsBox;  // slots before the first tile's that nobod
 constexpr int kRsMaxRows = 8;
 constexpr int kRsMaxWarps = 15;   // 136 registers a thread
 
-// Launch number (part of every message's pass number) and arrivals of the current launch.
+// Number of the next launch (part of every message's pass number), arrivals of the current launch or barrier.
 struct RsCtl {
   unsigned long long epoch;
   unsigned int ticket;
-  unsigned int pad;
+  unsigned int go;  // passes of a grid barrier (k_resident_sor)
 };
 
 struct RsArgs {
@@ -304,12 +304,19 @@ struct RsAddr {
   unsigned x, o, oe, oo, cls;
 };
 
+// What a pass with relaxation and residual sums (SOR) needs beside the rest: omega, RN(1/omega), the lane that
+// keeps the sum of row 0, the sums kept.
+struct RsSor {
+  double omega, romega, sum;
+  int at;
+};
+
 // The update of a row of the pair of planes (D: distance of the row).  The two planes are each other's
 // z-neighbours, which saves two of the loads, and two independent chains of dependent FP64 operations.
-template <int R, int D, bool ODD>
+template <int R, int D, bool ODD, bool SOR>
 __device__ __forceinline__ void rs_row(const RsAddr& a, unsigned tab, unsigned oa, unsigned cl, unsigned& cur,
                                        RsCoef (&k)[2], double om0, double oc0, double on0, double om1, double oc1,
-                                       double on1, double b0, double b1, double& n0, double& n1) {
+                                       double on1, double b0, double b1, double& n0, double& n1, RsSor& sor) {
   constexpr int PL = 2 * R * kRsRowPitch * 8;
   const double ot0 = lds<D>(ODD ? a.oo : a.oe), ot1 = lds<D + PL>(ODD ? a.oe : a.oo);
   const double z0 = lds<D - PL>(a.o), z1 = lds<D + 2 * PL>(a.o);
@@ -326,10 +333,35 @@ __device__ __forceinline__ void rs_row(const RsAddr& a, unsigned tab, unsigned o
       else q0 = q;
     }
   }
-  n0 = add(p0, sub(q0, p0));
-  n1 = add(p1, sub(q1, p1));
-  sts<D>(a.x, n0);
-  sts<D + PL>(a.x, n1);
+  if constexpr (!SOR) {
+    n0 = add(p0, sub(q0, p0));
+    n1 = add(p1, sub(q1, p1));
+    sts<D>(a.x, n0);
+    sts<D + PL>(a.x, n1);
+  } else {
+    // cells without a class keep what they have: a guard of an isothermal face is a neighbour like any other
+    const double d0 = sub(q0, p0), d1 = sub(q1, p1);
+    n0 = cl & 0xffffu ? add(p0, mul(sor.omega, d0)) : p0;
+    n1 = cl >> 16 ? add(p1, mul(sor.omega, d1)) : p1;
+    sts<D>(a.x, n0);
+    sts<D + PL>(a.x, n1);
+    // the residual of rb_pass_column; cx- is cxa in both parities of the row if oa is 0 (first plane)
+    const double g0 = mul(add(k[0].dd, mul(sor.omega, add(add(oa ? k[0].cxb : k[0].cxa, k[0].cym), k[0].czm))), d0);
+    const double g1 = mul(add(k[1].dd, mul(sor.omega, add(add(oa ? k[1].cxa : k[1].cxb, k[1].cym), k[1].czm))), d1);
+    double r0 = div_by(g0, sor.omega, sor.romega), r1 = div_by(g1, sor.omega, sor.romega);
+    if (div_bad(g0) || div_bad(g1)) {
+#pragma unroll 1
+      for (int w = 0; w < 2; ++w) {
+        const double r = div_fix(w ? g1 : g0, sor.omega, sor.romega, w ? r1 : r0);
+        if (w) r1 = r;
+        else r0 = r;
+      }
+    }
+    double v = add(cl & 0xffffu ? mul(r0, r0) : 0.0, cl >> 16 ? mul(r1, r1) : 0.0);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+    if (((int)threadIdx.x & 31) == sor.at + D / (kRsRowPitch * 8)) sor.sum = v;
+  }
 }
 
 template <int I, int N, typename F>
@@ -348,11 +380,11 @@ __device__ __forceinline__ void rs_each(F& f) {
 // pitches row and plane), loaded two rows ahead of its use; f and l are those of the first and last row.
 // (A cell without a class may get anything finite for b: its row of the table, zeros with dd = 1 and y = 0,
 // makes it 0.)
-template <int R, bool BS, typename Mid>
+template <int R, bool BS, bool SOR, typename Mid>
 __device__ __forceinline__ bool rs_rows(RsAddr a, unsigned tab, unsigned oa, unsigned bs, const double* bv, int row,
                                         int plane, double (&f)[2], double (&l)[2], RsCoef (&k)[2], unsigned& cur,
                                         const RsMsg& m, ulonglong2* box, bool to_lo, bool to_hi, unsigned seq,
-                                        Mid mid) {
+                                        RsSor& sor, Mid mid) {
   constexpr int P = kRsRowPitch * 8, PL = 2 * R * P, L = R - 1, BP = 2 * R * 256;
   double n0, n1, om0, om1, oc0, oc1, b0, b1, c0, c1;
   if (!BS && R > 2) {
@@ -368,7 +400,8 @@ __device__ __forceinline__ bool rs_rows(RsAddr a, unsigned tab, unsigned oa, uns
     f[0] = lds<0>(bs);
     f[1] = lds<BP>(bs);
   }
-  rs_row<R, 0, false>(a, tab, oa, ldsu<0>(a.cls), cur, k, m.vlo[0], om0, oc0, m.vlo[1], om1, oc1, f[0], f[1], n0, n1);
+  rs_row<R, 0, false, SOR>(a, tab, oa, ldsu<0>(a.cls), cur, k, m.vlo[0], om0, oc0, m.vlo[1], om1, oc1, f[0], f[1], n0, n1,
+                            sor);
   if (to_lo) {
     msg_store(box, n0, seq);
     msg_store(box + 2 * kRsBox, n1, seq);
@@ -383,9 +416,9 @@ __device__ __forceinline__ bool rs_rows(RsAddr a, unsigned tab, unsigned oa, uns
       l[0] = lds<L * 256>(bs);
       l[1] = lds<L * 256 + BP>(bs);
     }
-    rs_row<R, L * P, (L & 1) != 0>(a, tab, oa, ldsu<L * 128>(a.cls), cur, k, lds<(L - 1) * P>(a.o), lds<L * P>(a.o),
+    rs_row<R, L * P, (L & 1) != 0, SOR>(a, tab, oa, ldsu<L * 128>(a.cls), cur, k, lds<(L - 1) * P>(a.o), lds<L * P>(a.o),
                                    m.vhi[0], lds<(L - 1) * P + PL>(a.o), lds<L * P + PL>(a.o), m.vhi[1], l[0], l[1],
-                                   n0, n1);
+                                   n0, n1, sor);
   }
   if (to_hi) {
     msg_store(box + 32, n0, seq);
@@ -411,7 +444,8 @@ __device__ __forceinline__ bool rs_rows(RsAddr a, unsigned tab, unsigned oa, uns
           c1 = bv[plane];
         }
       }
-      rs_row<R, r * P, (r & 1) != 0>(a, tab, oa, ldsu<r * 128>(a.cls), cur, k, om0, oc0, on0, om1, oc1, on1, u0, u1, n0, n1);
+      rs_row<R, r * P, (r & 1) != 0, SOR>(a, tab, oa, ldsu<r * 128>(a.cls), cur, k, om0, oc0, on0, om1, oc1, on1, u0, u1, n0, n1,
+                                               sor);
       om0 = oc0;
       om1 = oc1;
       oc0 = on0;
@@ -715,8 +749,9 @@ __global__ void __launch_bounds__(32 * kRsMaxWarps, 1) k_resident(const __grid_c
       ad.oe = ad.o + (par ? 8u : -8u);
       ad.oo = ad.o - (par ? 8u : -8u);
       ad.cls = a.cls + (c ? R * 128 : 0);
-      ok = rs_rows<R, BS>(ad, tab, par ? 0u : 16u, saddr(B + pl * BP + c * (R * 32) + lane), bv, 2 * g.HP, plane, f, l,
-                          cf, cur, m, a.box + c * kRsBox, n_lo, n_hi, seq, mid);
+      RsSor none;
+      ok = rs_rows<R, BS, false>(ad, tab, par ? 0u : 16u, saddr(B + pl * BP + c * (R * 32) + lane), bv, 2 * g.HP, plane, f, l,
+                          cf, cur, m, a.box + c * kRsBox, n_lo, n_hi, seq, none, mid);
       if (R > 2) rs_send_edges<R>(a, c, seq, rest);
     }
     rs_post(prog + warp + 1, n + 1);
@@ -901,6 +936,326 @@ __global__ void __launch_bounds__(32 * kRsMaxWarps, 1) k_resident(const __grid_c
       }
       finish_stage(VM == 1 ? kStageAlpha : kStageOmega, A.st, s[0], s[1]);
     }
+  }
+}
+
+// ------------------------------------------------------------------------------------------
+// solveSOR!'s passes (k_sor_pass) with theta on the chip: up to `sweeps` passes over both colours in one
+// cooperative launch.  The tiles, messages and row updates are k_resident's; theta comes from memory, guards
+// and masked cells included, and goes back at the end.  After each pass over both colours the tiles leave the
+// blocks' sums of k_sor_pass and meet; the last one to arrive adds them in its order and tests for the end.
+// What bounds it: the chain of row updates and messages of the two colour passes, then the chain of row sums,
+// barrier and test (about half of the time of a small grid).  A pass over both colours: 169x169x30 15.1 us
+// (two launches of k_sor_pass: 22.6), 72x70x30 10.2 us (14.9).
+// ------------------------------------------------------------------------------------------
+template <int R, int NP, bool BS>
+__global__ void __launch_bounds__(32 * kRsMaxWarps, 1)
+    k_resident_sor(const __grid_constant__ RsArgs A, double omega, double romega, int sweeps,
+                   cudaGraphConditionalHandle hc, int use_cond) {
+  extern __shared__ double sh[];
+  __shared__ unsigned prog[kRsMaxWarps + 2];
+  __shared__ int am_last, ended;
+  __shared__ double red[16];
+  // Fail-safe loop bound: every launch first ends the loop, before any test; only the finisher of a pass
+  // (which runs after block 0 has arrived) can continue it.
+  if (blockIdx.x == 0 && threadIdx.x == 0) set_cond(hc, use_cond, 0);
+  if (A.st->stop || ld_relaxed_s32(A.err)) return;  // the same for every block
+  const Geo& g = A.op.g;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int tile = blockIdx.x, xb = tile % A.nxb, tj = tile / A.nxb;
+  const int NZ = g.NZ, j0 = 1 + tj * R, p = xb * 32 + lane;
+  constexpr int P = kRsRowPitch, CP = R * P, PL = 2 * CP, BP = 2 * R * 32, KP = 2 * R * 32;
+  double* X = sh + PL;
+  double* T = sh + rs_x_elems(R, NZ);
+  double* B = T + kRsTabRow * A.ntab;
+  unsigned* K = reinterpret_cast<unsigned*>(B + (BS ? (NZ + 1) / 2 * 2 * BP : 0));
+  const unsigned long long epoch = A.ctl->epoch;
+  const unsigned seq0 = (unsigned)epoch * 16u;
+  unsigned gen = ld_relaxed_u32(&A.ctl->go) & ~1u;
+  const bool n_lo = tj > 0, n_hi = tj + 1 < A.ntj, n_xm = xb > 0, n_xp = xb + 1 < A.nxb;
+  const int rows = min(R, g.NY - j0 + 1);
+  const unsigned tab = saddr(T);
+  const bool par0 = (1 + j0 + 1) & 1;
+  const int NZe = (NZ + 1) & ~1;
+  auto box_of = [&](int t, int pl) { return A.box + (size_t)(t * NZe + pl) * (2 * kRsBox); };
+  auto pair_at = [&](int pl0) {
+    RsPair a;
+    const ulonglong2* zero = A.box - kRsZero;
+    a.box = box_of(tile, pl0) + lane;
+    a.mlo = n_lo ? ~0u : 0u;
+    a.mhi = n_hi ? ~0u : 0u;
+    // beside the first and the last row of the grid: boxes that hold the guards' theta
+    a.lo = box_of(n_lo ? tile - A.nxb : (int)gridDim.x + xb, pl0) + 32 + lane;
+    a.hi = box_of(n_hi ? tile + A.nxb : (int)gridDim.x + A.nxb + xb, pl0) + lane;
+    const bool e = (1 + 1 + j0 + lane + pl0 + 1) & 1;
+    const bool xa = lane < R && (e ? n_xp : n_xm), xb = lane < R && (e ? n_xm : n_xp);
+    a.mxa = xa ? ~0u : 0u;
+    a.mxb = xb ? ~0u : 0u;
+    a.xa = xa ? box_of(e ? tile + 1 : tile - 1, pl0) + 64 + lane : zero;
+    a.xb = xb ? box_of(e ? tile - 1 : tile + 1, pl0) + 64 + lane : zero;
+    a.x = saddr(X + pl0 * PL + 1 + lane);
+    a.edge = saddr(X + pl0 * PL + (lane < R ? lane : 0) * P);
+    a.pad = e ? 264u : 0u;
+    a.cls = saddr(K + (pl0 / 2) * KP + lane);
+    return a;
+  };
+  auto inside = [&](int pl0, int r, int c, int w) {
+    const int i = 2 * p + (((1 + j0 + r + pl0 + w + 1) & 1) ^ c);
+    return pl0 + w < NZ && r < rows && p < g.HN && i >= 1 && i <= g.NX;
+  };
+  auto where = [&](int pl0, int r, int c, int w) { return g.row(c, j0 + r, pl0 + w + 1) + p; };
+  // theta of any cell, guards and masked cells included (0 beyond the guards)
+  auto theta = [&](int c, int j, int k) {
+    return p < g.HN && j <= g.NY + 1 && k <= NZ + 1 ? __ldcg(A.xx + g.row(c, j, k) + p) : 0.0;
+  };
+
+  // ---- the tile's table, theta, classes, b; theta of colour 1 to the neighbours --------------------------
+  if (threadIdx.x < kRsTabRow) T[threadIdx.x] = threadIdx.x == 8 ? 1.0 : 0.0;
+  {
+    const int n = A.count[tile];
+    const uint16_t* list = A.list + (size_t)tile * kRsMaxTab;
+    const double2* src = reinterpret_cast<const double2*>(A.op.ctab);
+    for (int q = threadIdx.x; q < 4 * n; q += blockDim.x) {
+      const double2 v = __ldg(src + 4 * (int)__ldg(list + (q >> 2)) + (q & 3));
+      double2* t = reinterpret_cast<double2*>(T) + 5 * (1 + (q >> 2));
+      t[(q & 3) + ((q & 3) > 0)] = v;
+      if ((q & 3) == 0) t[1] = make_double2(v.y, v.x);
+    }
+  }
+  if (threadIdx.x == 0) {
+    prog[0] = prog[nw + 1] = ~0u;
+    if (tile == 0) A.st->passes += 1;
+  }
+  if (lane == 0) prog[warp + 1] = 0u;
+  const int NZx = (NZ + 1) / 2 * 2;
+  for (int rc = warp; rc < 2 * R; rc += nw) {  // the planes below the first and above the last pair
+    X[-PL + rc * P + 1 + lane] = theta(rc / R, j0 + rc % R, 0);
+    X[NZx * PL + rc * P + 1 + lane] = theta(rc / R, j0 + rc % R, NZx + 1);
+  }
+#pragma unroll 1
+  for (int np = 0; np < NP; ++np) {
+    const int pl0 = (warp * NP + np) * 2;
+    if (pl0 >= NZ) break;
+    const RsPair a = pair_at(pl0);
+#pragma unroll 1
+    for (int r = 0; r < R; ++r) {
+      unsigned cl[4];
+#pragma unroll
+      for (int cw = 0; cw < 4; ++cw) {
+        const int c = cw >> 1, w = cw & 1;
+        const bool in = inside(pl0, r, c, w);
+        const double t = theta(c, j0 + r, pl0 + w + 1);
+        cl[cw] = in ? __ldg(A.lcls + where(pl0, r, c, w)) : 0u;
+        double* x = X + (pl0 + w) * PL + c * CP + r * P + 1 + lane;
+        x[0] = t;
+        if (lane == 0) x[-1] = 0.0;
+        if (lane == 31) x[1] = 0.0;
+        if (BS) B[(pl0 + w) * BP + (c * R + r) * 32 + lane] = cl[cw] ? __ldg(A.v + where(pl0, r, c, w)) : 1.0;
+        if (c == 1 && r == 0 && n_lo) msg_store(a.box + kRsBox + w * 2 * kRsBox, t, seq0);
+        if (c == 1 && r == R - 1 && n_hi) msg_store(a.box + kRsBox + w * 2 * kRsBox + 32, t, seq0);
+      }
+      unsigned* kr = K + (pl0 / 2) * KP + r * 32 + lane;
+      kr[0] = cl[0] | (cl[1] << 16);
+      kr[R * 32] = cl[2] | (cl[3] << 16);
+    }
+#pragma unroll
+    for (int cw = 0; cw < 4; ++cw) {
+      const int c = cw >> 1, w = cw & 1, at = c * kRsBox + w * 2 * kRsBox;
+      if (!n_lo) msg_store(const_cast<ulonglong2*>(a.lo) + at, theta(c, j0 - 1, pl0 + w + 1), 0u);
+      if (!n_hi) msg_store(const_cast<ulonglong2*>(a.hi) + at, theta(c, j0 + R, pl0 + w + 1), 0u);
+    }
+    rs_send_edges<R>(a, 1, seq0, lane < R);
+  }
+  __syncthreads();
+  rs_post(prog + warp + 1, 1u);
+
+  bool ok = true;
+  RsMsg m;
+  RsCoef cf[2];
+#pragma unroll
+  for (int w = 0; w < 2; ++w) {
+    cf[w].cxa = cf[w].cxb = cf[w].cym = cf[w].cyp = cf[w].czm = cf[w].czp = cf[w].y = 0.0;
+    cf[w].dd = 1.0;
+  }
+  unsigned cur = 0xffffffffu;
+  const bool ends = lane == 0 || lane == R - 1, rest = lane < R && !ends;
+  RsPair a = pair_at(warp * NP * 2);
+  RsSor sor;
+  sor.omega = omega;
+  sor.romega = romega;
+  const int gy = (g.NY + kBY - 1) / kBY, nb = A.nxb * gy * ((NZ + 1) / 2);
+#pragma unroll 1
+  for (unsigned n = 1;; ++n) {
+    const int c = (n - 1) & 1;
+    const unsigned seq = seq0 + n;
+    const bool par = par0 ^ (c != 0);
+    double f[2], l[2];
+    const double* bv;
+    auto first_b = [&](int pl) {
+      bv = A.v + g.row(c, j0, pl + 1) + p;
+      const int pp = pl + 1 < NZ ? (int)g.plane : 0;
+      f[0] = bv[0];
+      f[1] = bv[pp];
+      if (R > 1) {
+        l[0] = bv[(R - 1) * 2 * g.HP];
+        l[1] = bv[(R - 1) * 2 * g.HP + pp];
+      }
+      return pp;
+    };
+    int plane = 0;
+    if (NP == 1) {
+      m.fetch(a, c ^ 1);
+      if (!BS) plane = first_b(warp * 2);
+    }
+    rs_turn(cf);
+    ok = rs_wait_planes(prog + warp, prog + warp + 2, n, A);
+    // a warp has at most two pairs: their sums one after the other
+    double sums[NP];
+#pragma unroll
+    for (int np = 0; np < NP; ++np) {
+      sums[np] = 0.0;
+      const int pl = (warp * NP + np) * 2;
+      if (pl >= NZ || !ok) continue;
+      if (NP > 1) {
+        a = pair_at(pl);
+        m.fetch(a, c ^ 1);
+        if (!BS) plane = first_b(pl);
+      }
+      ok = rs_wait(m, a, c ^ 1, seq - 1, ends ? ~0u : 0u, A);
+      if (!ok) continue;
+      rs_put_edges<R>(m, a, c ^ 1, ends);
+      if (R > 2 && __any_sync(kFull, m.edges_missing(a, c ^ 1, seq - 1, rest ? ~0u : 0u))) m.fetch_edges(a, c ^ 1);
+      auto mid = [&] {
+        rs_send_edges<R>(a, c, seq, ends);
+        if (R <= 2) return true;
+        if (!rs_wait_edges(m, a, c ^ 1, seq - 1, rest ? ~0u : 0u, A)) return false;
+        rs_put_edges<R>(m, a, c ^ 1, rest);
+        return true;
+      };
+      RsAddr ad;
+      ad.x = a.x + (c ? CP * 8 : 0);
+      ad.o = a.x + (c ? 0 : CP * 8);
+      ad.oe = ad.o + (par ? 8u : -8u);
+      ad.oo = ad.o - (par ? 8u : -8u);
+      ad.cls = a.cls + (c ? R * 128 : 0);
+      sor.sum = 0.0;
+      sor.at = 0;
+      ok = rs_rows<R, BS, true>(ad, tab, par ? 0u : 16u, saddr(B + pl * BP + c * (R * 32) + lane), bv, 2 * g.HP, plane,
+                                f, l, cf, cur, m, a.box + c * kRsBox, n_lo, n_hi, seq, sor, mid);
+      sums[np] = sor.sum;
+      if (R > 2) rs_send_edges<R>(a, c, seq, rest);
+      // lane r has row r's sum
+      if (lane < rows)
+        msg_store(A.rowsum + ((size_t)c * nb + xb + A.nxb * (((tj * R + lane) >> 3) + gy * (pl / 2))) * 8 +
+                      ((tj * R + lane) & 7),
+                  sums[np], seq);
+    }
+    rs_post(prog + warp + 1, n + 1);
+    if (ok && c == 0) continue;
+
+    // ---- after both colours: k_sor_pass's block sums, by the tile that holds a group's first row --------
+    const int group = (tj * R + 7) >> 3;
+    if (group * 8 < tj * R + R && group * 8 < g.NY) {
+#pragma unroll 1
+      for (int np = 0; np < NP; ++np) {
+        const int pl = (warp * NP + np) * 2;
+        if (pl >= NZ || !ok) break;
+        const size_t id = (size_t)(lane >> 3) * nb + xb + A.nxb * (group + gy * (pl / 2));  // lane: colour * 8 + row
+        const unsigned want = (lane >> 3) ? seq : seq - 1;
+        const ulonglong2* src = lane < 16 && group * 8 + (lane & 7) < g.NY ? A.rowsum + id * 8 + (lane & 7) : nullptr;
+        double v = 0.0;
+        unsigned sv = want;
+        if (src) msg_load(src, v, sv);
+        const long long t0 = clock64();
+        while (!__all_sync(kFull, sv == want)) {
+          if (sv != want) msg_load(src, v, sv);
+          if (__all_sync(kFull, sv == want)) break;
+          if (rs_give_up(t0, A)) {
+            ok = false;
+            break;
+          }
+        }
+        v += __shfl_down_sync(kFull, v, 4);
+        v += __shfl_down_sync(kFull, v, 2);
+        v += __shfl_down_sync(kFull, v, 1);
+        if (lane == 0 || lane == 8) A.partials[id] = v;
+      }
+    }
+    // ---- every block meets; the last one tests for the end -------------------------------------------------
+    if (__syncthreads_or(!ok)) return;
+    if (threadIdx.x == 0) {
+      __threadfence();
+      am_last = atomicAdd(&A.ctl->ticket, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    gen += 2;  // the lowest bit: the solve has ended
+    bool good = true;
+    if (am_last) {
+      __threadfence();
+      // ordered_sum and block_sum of k_sor_pass's 256 threads
+      for (int vw = warp; vw < 16; vw += nw) {
+        const double* src = A.partials + (size_t)(vw >> 3) * nb;
+        double acc = 0.0;
+        for (int b0 = (vw & 7) * 32 + lane; b0 < nb; b0 += 256 * 8) {
+          double t[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) t[u] = b0 + 256 * u < nb ? __ldcg(src + b0 + 256 * u) : 0.0;
+#pragma unroll
+          for (int u = 0; u < 8; ++u) acc += t[u];
+        }
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(kFull, acc, o);
+        if (lane == 0) red[vw] = acc;
+      }
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        auto tree8 = [&](const double* v) {
+          return ((v[0] + v[4]) + (v[2] + v[6])) + ((v[1] + v[5]) + (v[3] + v[7]));
+        };
+        finish_stage(kStageSorHalf, A.st, tree8(red), 0.0);
+        finish_stage(kStageSorIter, A.st, tree8(red + 8), 0.0);
+        const bool stop = A.st->stop;
+        if (n >= 2u * (unsigned)sweeps && !stop) set_cond(hc, use_cond, A.st->passes <= A.st->maxItr + 1);
+        A.ctl->ticket = 0;
+        A.ctl->epoch = epoch + n / 16u + 1;
+        ended = stop;
+        asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&A.ctl->go), "r"(gen | (stop ? 1u : 0u)) : "memory");
+      }
+    } else if (threadIdx.x == 0) {
+      const long long t0 = clock64();
+      for (;;) {
+        unsigned v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&A.ctl->go) : "memory");
+        if ((v & ~1u) == gen) {
+          ended = v & 1u;
+          break;
+        }
+        const bool late = clock64() - t0 > A.limit;
+        if (late || ld_relaxed_s32(A.err)) {
+          if (late) {
+            atomicExch(A.err, 1);
+            A.st->stop = 1;
+            A.st->reason = kTimeout;
+          }
+          good = false;
+          break;
+        }
+      }
+    }
+    if (__syncthreads_or(!good)) return;
+    if (ended || n >= 2u * (unsigned)sweeps) break;
+  }
+
+  // ---- theta back to memory ------------------------------------------------------------------------------
+#pragma unroll 1
+  for (int np = 0; np < NP; ++np) {
+    const int pl0 = (warp * NP + np) * 2;
+    if (pl0 >= NZ) break;
+#pragma unroll 1
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int cw = 0; cw < 4; ++cw)
+        if (inside(pl0, r, cw >> 1, cw & 1))
+          A.xx[where(pl0, r, cw >> 1, cw & 1)] = X[(pl0 + (cw & 1)) * PL + (cw >> 1) * CP + r * P + 1 + lane];
   }
 }
 

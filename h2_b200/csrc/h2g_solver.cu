@@ -515,6 +515,7 @@ static int launch_coop(Solver* s, cudaStream_t cs, const OpParams<double>& op, d
 }
 // ---- resident preconditioner (k_resident) ------------------------------------------------------
 const void* resident_kernel(int R, int np, int vm);
+const void* resident_sor_kernel(int R, int np);
 cudaError_t launch_tile_classes(cudaStream_t st, const Geo& g, const uint16_t* cls, uint16_t* lcls, uint16_t* list,
                                 int* count, int R, int nxb, int ntj);
 static bool resident_b_shared(const ResidentPlan& pl) { return pl.R <= (pl.np == 1 ? 5 : 2); }
@@ -591,8 +592,10 @@ static ResidentPlan resident_plan(const Solver* s) {
 // return: a tile has more classes than fit beside its x and b.
 static int resident_prepare(Solver* s, ResidentPlan& pl) {
   const Geo& g = s->g;
-  // room for every split: a handle may run with all SMs in one call and a share of them in the next
-  const size_t box = sizeof(ulonglong2) * ((size_t)s->num_sms * ((g.NZ + 1) & ~1) * 2 * kRsBox + kRsZero);
+  // room for every split (a handle may run with all SMs in one call and a share of them in the next) and for
+  // the guards' rows of k_resident_sor
+  const size_t box =
+      sizeof(ulonglong2) * ((size_t)(s->num_sms + 2 * pl.nxb) * ((g.NZ + 1) & ~1) * 2 * kRsBox + kRsZero);
   if (!s->rs_ctl) {
     const size_t nb = (size_t)pl.nxb * ((g.NY + kBY - 1) / kBY) * g.NZ;
     CK(cudaMalloc(&s->rs_box, box));
@@ -628,6 +631,9 @@ static int resident_prepare(Solver* s, ResidentPlan& pl) {
     CK(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device));
     s->rs_fits = s->rs_ntab <= kRsMaxTab && s->rs_smem + 512 <= (size_t)most;
     if (s->rs_fits)
+      CK(cudaFuncSetAttribute(resident_sor_kernel(pl.R, pl.np), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              most - 512));
+    if (s->rs_fits)
       for (int vm = 0; vm < 3; ++vm)
         CK(cudaFuncSetAttribute(resident_kernel(pl.R, pl.np, vm), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 most - 512));
@@ -637,16 +643,11 @@ static int resident_prepare(Solver* s, ResidentPlan& pl) {
   return H2G_OK;
 }
 
-static int launch_resident(Solver* s, cudaStream_t cs, const OpParams<double>& op, int vm, double* xx, double* v,
-                           const double* r, const double* q, double* y, const double* u, SolverState* st) {
-  RsArgs a;
+static RsArgs resident_args(const Solver* s, const OpParams<double>& op, double* xx, double* v, SolverState* st) {
+  RsArgs a = {};
   a.op = op;
   a.xx = xx;
   a.v = v;
-  a.r = r;
-  a.q = q;
-  a.y = y;
-  a.u = u;
   a.st = st;
   a.rowsum = s->rs_rowsum;
   a.partials = s->partials;
@@ -660,9 +661,13 @@ static int launch_resident(Solver* s, cudaStream_t cs, const OpParams<double>& o
   a.limit = s->wait_limit;
   a.nxb = s->rs.nxb;
   a.ntj = s->rs.ntj;
+  return a;
+}
+
+static int launch_tiles(Solver* s, cudaStream_t cs, const void* kernel, void** args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(s->rs.blocks());
-  cfg.blockDim = dim3(s->rs.threads(op.g.NZ));
+  cfg.blockDim = dim3(s->rs.threads(s->g.NZ));
   cfg.dynamicSmemBytes = s->rs_smem;
   cfg.stream = cs;
   cudaLaunchAttribute attr[1];
@@ -670,11 +675,33 @@ static int launch_resident(Solver* s, cudaStream_t cs, const OpParams<double>& o
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  void* args[] = {&a};
-  if (cudaLaunchKernelExC(&cfg, resident_kernel(s->rs.R, s->rs.np, vm), args) != cudaSuccess)
+  if (cudaLaunchKernelExC(&cfg, kernel, args) != cudaSuccess)
     return fail(H2G_CUDA_ERROR, "cooperative launch of %d blocks failed: %s", s->rs.blocks(),
                 cudaGetErrorString(cudaGetLastError()));
   return H2G_OK;
+}
+
+static int launch_resident(Solver* s, cudaStream_t cs, const OpParams<double>& op, int vm, double* xx, double* v,
+                           const double* r, const double* q, double* y, const double* u, SolverState* st) {
+  RsArgs a = resident_args(s, op, xx, v, st);
+  a.r = r;
+  a.q = q;
+  a.y = y;
+  a.u = u;
+  void* args[] = {&a};
+  return launch_tiles(s, cs, resident_kernel(s->rs.R, s->rs.np, vm), args);
+}
+
+// Passes of solveSOR! in one launch: the tiles' set-up (theta, table, classes, b) is paid once for them.
+constexpr int kSorSweeps = 32;
+
+static int launch_resident_sor(Solver* s, cudaStream_t cs, const OpParams<double>& op, double omega, SolverState* st,
+                               cudaGraphConditionalHandle hc, int use_cond) {
+  RsArgs a = resident_args(s, op, s->th, s->b, st);
+  double romega = 1.0 / omega;
+  int sweeps = kSorSweeps;
+  void* args[] = {&a, &omega, &romega, &sweeps, &hc, &use_cond};
+  return launch_tiles(s, cs, resident_sor_kernel(s->rs.R, s->rs.np), args);
 }
 
 static bool use_coop(const Solver* s) { return s->rb_coop && !s->coop_barred && !s->rb_fused; }
@@ -1330,6 +1357,13 @@ static int make_loop_graph(Solver* s, SolveGraph& G, Body body) {
   return H2G_OK;
 }
 
+static void sign_resident(const Solver* s, std::vector<unsigned char>& sig) {
+  const unsigned char* d = reinterpret_cast<const unsigned char*>(&s->rs);
+  sig.insert(sig.end(), d, d + sizeof s->rs);
+  d = reinterpret_cast<const unsigned char*>(&s->rs_box);
+  sig.insert(sig.end(), d, d + sizeof s->rs_box);
+}
+
 template <typename T, typename TX, typename TP>
 static int get_graph(Solver* s, int kind, int smoother, const OpParams<T>& op, const OpParams<TP>& opM, TX* x,
                      SolverState* st, SolveGraph** out) {
@@ -1337,12 +1371,7 @@ static int get_graph(Solver* s, int kind, int smoother, const OpParams<T>& op, c
   SolveGraph& G = s->graphs[kind][resident ? (s->sm_share ? 3 : 2) : smoother ? 1 : 0];
   std::vector<unsigned char> sig = signature(op, opM, smoother, (const void*)x);
   sig.push_back(use_coop(s) ? 1 : 0);
-  if (resident) {
-    const unsigned char* d = reinterpret_cast<const unsigned char*>(&s->rs);
-    sig.insert(sig.end(), d, d + sizeof s->rs);
-    d = reinterpret_cast<const unsigned char*>(&s->rs_box);
-    sig.insert(sig.end(), d, d + sizeof s->rs_box);
-  }
+  if (resident) sign_resident(s, sig);
   if (G.exec && G.sig == sig) {
     *out = &G;
     return H2G_OK;
@@ -1877,6 +1906,17 @@ static int autotune(Solver* s);
 struct ResidentCall {
   Solver* s = nullptr;
   SmLease lease;
+  // solveSOR!: the relaxation's quotient by its reciprocal needs omega within 2^+-100 (div_by)
+  int begin_sor(Solver* solver, double omega) {
+    ResidentPlan pl = omega >= 0x1p-100 ? resident_plan(solver) : ResidentPlan();
+    if (pl.R)
+      if (int rc = resident_prepare(solver, pl)) return rc;
+    if (!pl.R) return H2G_OK;
+    s = solver;
+    lease.take(s, pl.blocks());
+    s->rs = pl;
+    return H2G_OK;
+  }
   int begin(Solver* solver, int smoother) {
     s = solver;
     ResidentPlan pl = smoother == H2G_SMOOTHER_GS ? resident_plan(s) : ResidentPlan();
@@ -1955,6 +1995,9 @@ static int solve_sor(Solver* s, double omega, double tol, int maxItr, int verbos
   const Geo& g = s->g;
   int rc = ensure_hist(s, maxItr);
   if (rc) return rc;
+  ResidentCall call;
+  if ((rc = call.begin_sor(s, omega))) return rc;
+  const bool resident = s->rs.R != 0;
   const OpParams<double> op = op_params<double>(s, s->t64);
   SolverState* st = s->st;
   if ((rc = prime_state(s, st, tol, maxItr, s->hist, maxItr))) return rc;
@@ -1962,23 +2005,31 @@ static int solve_sor(Solver* s, double omega, double tol, int maxItr, int verbos
   launch(s, k_res_sor, ag, blk, s->stream, op, (const double*)s->th, (const double*)s->b, omega, st, s->partials,
          (int)kStageSorInit);
   CKL();
-  SolveGraph& G = s->graphs[kGSor][0];
+  SolveGraph& G = s->graphs[kGSor][resident ? (s->sm_share ? 3 : 2) : 0];
   std::vector<unsigned char> sig(sizeof op + sizeof omega);
   memcpy(sig.data(), &op, sizeof op);
   memcpy(sig.data() + sizeof op, &omega, sizeof omega);
   sig.push_back(s->recip_ok ? 1 : 0);
+  if (resident) sign_resident(s, sig);
   if (!G.exec || G.sig != sig) {
+    int berr = H2G_OK;
     rc = make_loop_graph(s, G, [&](cudaStream_t cs, cudaGraphConditionalHandle hc, int use_cond) {
+      if (resident) {
+        berr = launch_resident_sor(s, cs, op, omega, st, hc, use_cond);
+        return;
+      }
       // the quotients by reciprocals need dd and omega within 2^+-100 (div_by)
       if (op.cls && op.cls_dd && s->recip_ok && omega >= 0x1p-100)
         sor_passes<2, true>(s, cs, op, rg, blk, omega, st, hc, use_cond);
       else if (op.cls) sor_passes<2, false>(s, cs, op, rg, blk, omega, st, hc, use_cond);
       else sor_passes<1, false>(s, cs, op, rg, blk, omega, st, hc, use_cond);
     });
+    if (rc == H2G_OK && berr != H2G_OK) G.reset();
     if (rc) return rc;
+    if (berr) return berr;
     G.sig = sig;
   }
-  if ((rc = run_graph(s, &G, st, maxItr, 1))) return rc;
+  if ((rc = run_graph(s, &G, st, maxItr, resident ? kSorSweeps : 1))) return rc;
   CK(cudaMemcpyAsync(s->st_host, st, sizeof(SolverState), cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));
   SolverState fin = *s->st_host;
@@ -1990,13 +2041,23 @@ static int solve_sor(Solver* s, double omega, double tol, int maxItr, int verbos
   }
   if (verbose) print_log(fin, hh.data(), nh, fin.converged);
   if (out) {
-    out->launches = 2 + 2LL * std::max(1, fin.itr);
+    const int its = std::max(1, fin.itr);
+    out->launches = 2 + (resident ? (its + kSorSweeps - 1) / kSorSweeps : 2LL * its);
     out->isconverged = fin.converged;
     out->itr = fin.itr;
     out->outer = 0;
     out->status = status_of(fin);
     out->res0 = fin.res0;
     out->res = fin.res;
+  }
+  if (resident) {
+    if (const int e = sweep_status(s)) {  // a bounded wait ran out: theta is that of the last whole launch
+      if (out) {
+        out->status = e;
+        out->isconverged = 0;
+      }
+      return e;
+    }
   }
   return status_of(fin);
 }
@@ -3125,7 +3186,7 @@ int h2g_batch_solve(int n, h2g_solver* const* hs, int method, double tol, int ma
   for (int q = 0; q < n; ++q) {
     const Solver* s = S(hs[q]);
     order[q] = q;
-    const h2g::ResidentPlan pl = method != 2 && smoother == H2G_SMOOTHER_GS ? h2g::resident_plan(s) : h2g::ResidentPlan();
+    const h2g::ResidentPlan pl = method == 2 || smoother == H2G_SMOOTHER_GS ? h2g::resident_plan(s) : h2g::ResidentPlan();
     if (pl.R && nt > 1) rank[q] = pl.blocks() > s->sm_share ? 0 : 1;
   }
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) {

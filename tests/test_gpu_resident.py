@@ -190,3 +190,47 @@ def test_batch_shares(oracle, threads):
             assert g[:2] == ref[:2] and np.array_equal(g[2], ref[2])
     for s in hs:
         s.close()
+
+
+@pytest.mark.parametrize("n", SIZES, ids=lambda n: "x".join(map(str, n)))
+def test_sor_identical(oracle, n):
+    """solveSOR! with theta on the chip: field and residual history of the separate passes, bit for bit, for
+    passes within a launch, a whole launch and more, and where the last test ends the solve."""
+    prob = mode3_model(oracle, *n)
+    s, ref = make_solver(prob), make_solver(prob)
+    ref.set_tuning(8, 2)
+    for omega, passes, tol in ((1.5, 1, 0.0), (1.0, 32, 0.0), (1.5, 71, 0.0), (1.0, 60, 0.5)):
+        out = []
+        for q in (s, ref):
+            q.set_theta(prob.wk["theta"])
+            hist = np.zeros(passes)
+            st, res = q.sor(omega=omega, tol=tol, maxItr=passes, hist=hist)
+            out.append((st, res.itr, res.res0, res.res, hist, q.get_theta()))
+        assert res.launches == 2 + 2 * res.itr
+        assert out[0][:4] == out[1][:4]
+        assert np.array_equal(out[0][4], out[1][4]) and np.array_equal(out[0][5], out[1][5])
+    s.set_wait_limit(0)
+    res = L.Result()
+    assert L.load().h2g_sor(s.h, 1.0, 0.0, 20, 0, None, ctypes.byref(res)) == L.H2G_TIMEOUT
+    s.set_wait_limit(2_000_000_000)
+    s.set_theta(prob.wk["theta"])
+    s.sor(omega=1.0, tol=0.5, maxItr=60)
+    assert np.array_equal(s.get_theta(), out[0][5])
+    s.close()
+    ref.close()
+
+
+@pytest.mark.parametrize("grid", GRIDS, ids=["x".join(map(str, g)) for g in GRIDS])
+def test_sor_boxes(oracle, grid):
+    prob = box_problem(oracle, *grid, seed=sum(grid) + 3)
+    s, ref = make_solver(prob), make_solver(prob)
+    ref.set_tuning(8, 2)
+    out = []
+    for q in (s, ref):
+        hist = np.zeros(40)
+        st, res = q.sor(omega=1.3, tol=0.0, maxItr=40, hist=hist)
+        out.append((res.itr, hist, q.get_theta()))
+    assert out[0][0] == out[1][0]
+    assert np.array_equal(out[0][1], out[1][1], equal_nan=True) and np.array_equal(out[0][2], out[1][2], equal_nan=True)
+    s.close()
+    ref.close()
