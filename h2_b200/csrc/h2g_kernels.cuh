@@ -366,10 +366,9 @@ __device__ __forceinline__ void x_nbrs(T oc, int okc, int e, int lane, int p, in
 // returns the sum of the squared SOR residuals r = (dd + omega*(c_xm + c_ym + c_zm))*dp/omega of
 // the updated cells (rbsor_core!, NonUniform.jl:907-908); the preconditioner discards them and
 // skips the work.  With NP = 2 the two cells share the o-colour column loads.
-// RCP (FP64, class table): both quotients by their reciprocals, RN(1/dd) of the class row and romega = RN(1/omega).
-template <typename T, bool RES, int NP = 2, int DDM = 1, bool NC = true, bool RCP = false>
+template <typename T, bool RES, int NP = 2, int DDM = 1, bool NC = true>
 __device__ __forceinline__ double rb_pass_column(const OpParams<T>& op, T* x, const T* __restrict__ bb, int color,
-                                                 T omega, int lane, int p, int j, int k0, T romega = T(0)) {
+                                                 T omega, int lane, int p, int j, int k0) {
   const Geo& g = op.g;
   const int o = color ^ 1;
   const bool pok = p < g.HN;
@@ -449,25 +448,10 @@ __device__ __forceinline__ double rb_pass_column(const OpParams<T>& op, T* x, co
     }
     if (!has) continue;
     const T ss = nb_sum(c, xp[u], xm[u], yp[u], ym[u], col[u + 2], col[u]);
-    T q;
-    if constexpr (RCP) {
-      const T a = sub(ss, bv[u]);
-      q = div_by(a, c.dd, __ldg(op.ctab + 8 * cl[u] + 7));
-      if (div_bad(a)) q = dvd(a, c.dd);
-    } else {
-      q = gs_div(sub(ss, bv[u]), c.dd);
-    }
-    const T dp = sub(q, pp[u]);  // * m0 (= 1)
+    const T dp = sub(gs_div(sub(ss, bv[u]), c.dd), pp[u]);  // * m0 (= 1)
     x[ac] = relax(pp[u], omega, dp);
     if constexpr (RES) {
-      const T a = mul(add(c.dd, mul(omega, add(add(c.cxm, c.cym), c.czm))), dp);
-      T r;
-      if constexpr (RCP) {
-        r = div_by(a, omega, romega);
-        if (div_bad(a)) r = dvd(a, omega);
-      } else {
-        r = dvd(a, omega);
-      }
+      const T r = dvd(mul(add(c.dd, mul(omega, add(add(c.cxm, c.cym), c.czm))), dp), omega);
       acc = add(acc, mul((double)r, (double)r));
     }
   }
@@ -499,12 +483,13 @@ __global__ void __launch_bounds__(kBX * BY, ((DDM == 2 ? H2G_MINB_CLS : H2G_MINB
 // rbsor_core! with its residual (NonUniform.jl:848-915) for solveSOR! (NonUniform.jl:1004-1051): colour C updated
 // with relaxation omega.  Both colours leave their blocks' sums of r^2; the last block of colour 1 adds both in the
 // order of reduce_finish (kStageSorHalf, kStageSorIter): a finisher after colour 0 kept the next launch waiting for
-// a ticket and a sum that nobody needed yet.  With that and the two quotients of a cell by reciprocals (RCP) a pass
-// over both colours takes 22.6 us instead of 25.7 (169x169x30), 14.9 instead of 17.3 (72x70x30).  The colour-1 launch ends a WHILE-body pass: block 0 counts the pass
-// and ends the loop provisionally; only the finisher can continue it.
-template <bool COND, int DDM, int C, bool RCP>
+// a ticket and a sum that nobody needed yet.  A pass over both colours takes 44 us instead of 51 (281x281x30);
+// with the quotients by reciprocals, as k_resident_sor has them, it took 45.6: the loads set its pace, not the
+// divisions.  The colour-1 launch ends a WHILE-body pass: block 0 counts the pass and ends the loop
+// provisionally; only the finisher can continue it.
+template <bool COND, int DDM, int C>
 __global__ void __launch_bounds__(kThreads) k_sor_pass(OpParams<double> op, double* x,
-                                                       const double* __restrict__ bb, double omega, double romega,
+                                                       const double* __restrict__ bb, double omega,
                                                        SolverState* st, double* __restrict__ partials,
                                                        cudaGraphConditionalHandle hc, int use_cond) {
   pdl_enter();
@@ -517,7 +502,7 @@ __global__ void __launch_bounds__(kThreads) k_sor_pass(OpParams<double> op, doub
   const int j = 1 + blockIdx.y * kBY + threadIdx.y;
   const int k0 = 1 + 2 * blockIdx.z;
   double v[1] = {0.0};
-  if (j <= op.g.NY) v[0] = rb_pass_column<double, true, 2, DDM, true, RCP>(op, x, bb, C, omega, lane, p, j, k0, romega);
+  if (j <= op.g.NY) v[0] = rb_pass_column<double, true, 2, DDM>(op, x, bb, C, omega, lane, p, j, k0);
   __shared__ double sm[32][1], sm2[32][2];
   __shared__ int am_last;
   const int tid = threadIdx.x + kBX * threadIdx.y;

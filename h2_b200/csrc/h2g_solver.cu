@@ -230,6 +230,7 @@ struct Solver {
   int rs_ntab = 0;              // rows of the largest tile table (0: to be made)
   int rs_rows = 0;              // R of the split that the tables are for
   size_t rs_smem = 0;
+  int rs_most = 0;              // dynamic shared memory that the kernels may ask for
   bool rs_fits = false;
   // K right-hand sides on the handle's operator (h2g_create_multi): stacked vectors, K states
   int nrhs = 0;
@@ -630,13 +631,7 @@ static int resident_prepare(Solver* s, ResidentPlan& pl) {
     int most = 0;
     CK(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device));
     s->rs_fits = s->rs_ntab <= kRsMaxTab && s->rs_smem + 512 <= (size_t)most;
-    if (s->rs_fits)
-      CK(cudaFuncSetAttribute(resident_sor_kernel(pl.R, pl.np), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              most - 512));
-    if (s->rs_fits)
-      for (int vm = 0; vm < 3; ++vm)
-        CK(cudaFuncSetAttribute(resident_kernel(pl.R, pl.np, vm), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                most - 512));
+    s->rs_most = most - 512;
   }
   pl.ntab = s->rs_ntab;
   if (!s->rs_fits) pl.R = 0;
@@ -664,17 +659,19 @@ static RsArgs resident_args(const Solver* s, const OpParams<double>& op, double*
   return a;
 }
 
-static int launch_tiles(Solver* s, cudaStream_t cs, const void* kernel, void** args) {
+static int launch_tiles(Solver* s, cudaStream_t cs, const void* kernel, void** args, bool pdl) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(s->rs.blocks());
   cfg.blockDim = dim3(s->rs.threads(s->g.NZ));
   cfg.dynamicSmemBytes = s->rs_smem;
   cfg.stream = cs;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = s->pdl && pdl ? 2 : 1;
   if (cudaLaunchKernelExC(&cfg, kernel, args) != cudaSuccess)
     return fail(H2G_CUDA_ERROR, "cooperative launch of %d blocks failed: %s", s->rs.blocks(),
                 cudaGetErrorString(cudaGetLastError()));
@@ -689,7 +686,7 @@ static int launch_resident(Solver* s, cudaStream_t cs, const OpParams<double>& o
   a.y = y;
   a.u = u;
   void* args[] = {&a};
-  return launch_tiles(s, cs, resident_kernel(s->rs.R, s->rs.np, vm), args);
+  return launch_tiles(s, cs, resident_kernel(s->rs.R, s->rs.np, vm), args, true);
 }
 
 // Passes of solveSOR! in one launch: the tiles' set-up (theta, table, classes, b) is paid once for them.
@@ -701,7 +698,7 @@ static int launch_resident_sor(Solver* s, cudaStream_t cs, const OpParams<double
   double romega = 1.0 / omega;
   int sweeps = kSorSweeps;
   void* args[] = {&a, &omega, &romega, &sweeps, &hc, &use_cond};
-  return launch_tiles(s, cs, resident_sor_kernel(s->rs.R, s->rs.np), args);
+  return launch_tiles(s, cs, resident_sor_kernel(s->rs.R, s->rs.np), args, false);
 }
 
 static bool use_coop(const Solver* s) { return s->rb_coop && !s->coop_barred && !s->rb_fused; }
@@ -1912,6 +1909,8 @@ struct ResidentCall {
     if (pl.R)
       if (int rc = resident_prepare(solver, pl)) return rc;
     if (!pl.R) return H2G_OK;
+    CK(cudaFuncSetAttribute(resident_sor_kernel(pl.R, pl.np), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            solver->rs_most));
     s = solver;
     lease.take(s, pl.blocks());
     s->rs = pl;
@@ -1923,6 +1922,9 @@ struct ResidentCall {
     if (pl.R)
       if (int rc = resident_prepare(s, pl)) return rc;
     if (pl.R) {
+      for (int vm = 0; vm < 3; ++vm)
+        CK(cudaFuncSetAttribute(resident_kernel(pl.R, pl.np, vm), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                s->rs_most));
       if (!s->rb_tuned) s->ax_cls = true;  // CG's CalcAX: the class table, untimed
       lease.take(s, pl.blocks());
       s->rs = pl;
@@ -1968,18 +1970,17 @@ static int solve(Solver* s, bool cg, double tol, int maxItr, int smoother, int v
 // creation and set-up
 // ------------------------------------------------------------------------------------------
 // One rbsor! (colour 0, colour 1, each with its residual sum) with the coefficients from the key
-// tables (DDM 1) or the stencil-class table (DDM 2; RCP: its dd and omega have reciprocals for div_by).
-template <int DDM, bool RCP>
+// tables (DDM 1) or the stencil-class table (DDM 2).
+template <int DDM>
 static void sor_passes(Solver* s, cudaStream_t cs, const OpParams<double>& op, dim3 rg, dim3 blk, double omega,
                        SolverState* st, cudaGraphConditionalHandle hc, int use_cond) {
-  const double romega = 1.0 / omega;
-  launch(s, k_sor_pass<false, DDM, 0, RCP>, rg, blk, cs, op, s->th, (const double*)s->b, omega, romega, st, s->partials,
+  launch(s, k_sor_pass<false, DDM, 0>, rg, blk, cs, op, s->th, (const double*)s->b, omega, st, s->partials,
          hc, 0);
   if (use_cond)
-    launch(s, k_sor_pass<true, DDM, 1, RCP>, rg, blk, cs, op, s->th, (const double*)s->b, omega, romega, st, s->partials,
+    launch(s, k_sor_pass<true, DDM, 1>, rg, blk, cs, op, s->th, (const double*)s->b, omega, st, s->partials,
            hc, use_cond);
   else
-    launch(s, k_sor_pass<false, DDM, 1, RCP>, rg, blk, cs, op, s->th, (const double*)s->b, omega, romega, st,
+    launch(s, k_sor_pass<false, DDM, 1>, rg, blk, cs, op, s->th, (const double*)s->b, omega, st,
            s->partials, hc, use_cond);
 }
 
@@ -2009,7 +2010,6 @@ static int solve_sor(Solver* s, double omega, double tol, int maxItr, int verbos
   std::vector<unsigned char> sig(sizeof op + sizeof omega);
   memcpy(sig.data(), &op, sizeof op);
   memcpy(sig.data() + sizeof op, &omega, sizeof omega);
-  sig.push_back(s->recip_ok ? 1 : 0);
   if (resident) sign_resident(s, sig);
   if (!G.exec || G.sig != sig) {
     int berr = H2G_OK;
@@ -2018,11 +2018,8 @@ static int solve_sor(Solver* s, double omega, double tol, int maxItr, int verbos
         berr = launch_resident_sor(s, cs, op, omega, st, hc, use_cond);
         return;
       }
-      // the quotients by reciprocals need dd and omega within 2^+-100 (div_by)
-      if (op.cls && op.cls_dd && s->recip_ok && omega >= 0x1p-100)
-        sor_passes<2, true>(s, cs, op, rg, blk, omega, st, hc, use_cond);
-      else if (op.cls) sor_passes<2, false>(s, cs, op, rg, blk, omega, st, hc, use_cond);
-      else sor_passes<1, false>(s, cs, op, rg, blk, omega, st, hc, use_cond);
+      if (op.cls) sor_passes<2>(s, cs, op, rg, blk, omega, st, hc, use_cond);
+      else sor_passes<1>(s, cs, op, rg, blk, omega, st, hc, use_cond);
     });
     if (rc == H2G_OK && berr != H2G_OK) G.reset();
     if (rc) return rc;
