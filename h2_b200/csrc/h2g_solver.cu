@@ -566,8 +566,10 @@ class SmLease {
 // the handle's share of them.  A pass grows more slowly than its rows (its messages and barriers stay), so
 // two solves on halves beat two in turn on all: 120^2, 180^2 and 240^2 twice each, two threads, in turn 224 ms,
 // the first two on halves 192 ms (colour passes beside each other 218 ms).  A warp has one pair of
-// planes up to 30 planes (up to 8 rows: 240x240x30 takes 7, 140 tiles), two pairs up to 60 planes (4
-// rows).  Larger grids keep the separate launches, as do the grids without a class table or with tiles of
+// planes up to 30 planes (up to 8 rows: 240x240x30 takes 7, 140 tiles; 20x20 62.9 -> 47.4, 120x120 88 -> 64,
+// 240x240 216 -> 158 us an iteration), two pairs up to 60 planes (4 rows) if the grid fills the tiles: 70x70x60
+// (half of the positions, 1 row) 97 -> 86, 145x145x60 (74 %) 200 -> 179, but 80x80x60 (34 %) 103 -> 118, 100x100x60
+// (53 %) 116 -> 121.  Larger grids keep the separate launches, as do the grids without a class table or with tiles of
 // too many classes (resident_prepare), the FP32 smoother, and handles on which a launch shape, a
 // coefficient source or another form of the preconditioner was asked for.
 static ResidentPlan resident_plan(const Solver* s) {
@@ -584,7 +586,10 @@ static ResidentPlan resident_plan(const Solver* s) {
   for (int sms : {s->sm_share, s->num_sms})
     for (pl.R = 1; pl.R <= (pl.np == 1 ? kRsMaxRows : 4); ++pl.R) {
       pl.ntj = (g.NY + pl.R - 1) / pl.R;
-      if (pl.blocks() <= sms) return pl;
+      if (pl.blocks() > sms) continue;
+      // two pairs a warp: a pass takes twice as long, so most of the SMs' positions must be in the grid
+      if (pl.np == 2 && 100LL * g.NX * g.NY < (pl.R == 1 ? 50LL : 65LL) * sms * 64 * pl.R) break;
+      return pl;
     }
   return no;
 }

@@ -7,7 +7,8 @@ BOX = 72
 
 
 def plan(NX, NY, NZ, sms=148):
-    """resident_plan: (R, pairs of planes per warp, tiles along positions, tiles along rows) or None."""
+    """resident_plan: (R, pairs of planes per warp, tiles along positions, tiles along rows) or None; without its
+    rule on how full the tiles must be beyond 30 planes."""
     HN = (NX + 3) // 2
     nxb = (HN + 31) // 32
     np_ = 1 if NZ <= 30 else 2
