@@ -22,8 +22,8 @@
 // reader polls the 16 bytes until the number is the one it waits for.  There is no grid barrier and
 // no fence; one message is one trip through L2, about 1000 cycles.  Inside a tile a warp waits for the
 // warps of the planes below and above, not for the block.  A pass updates its first and last row
-// first, so that their messages travel while the rows between are updated.  One slot per cell and colour suffices: a cell is
-// overwritten a sweep later, by an update that needs the reader's value of the pass in between, which
+// first, so that their messages travel while the rows between are updated.  One slot per cell and colour
+// suffices: a cell is overwritten a sweep later, by an update that needs the reader's value of the pass in between, which
 // the reader made after reading the slot.  Every wait is bounded like the grid barriers'.
 //
 // Results are the bits of the separate launches: the same operations per cell, the same quotient (see
@@ -531,6 +531,9 @@ static __global__ void __launch_bounds__(256) k_tile_classes(Geo g, const uint16
 // VM 0: xx = M^-1 v.  VM 1: p = r + beta (p - omega q) in v, xx = M^-1 p, y = A xx, (y, u) ->
 // kStageAlpha.  VM 2: s = r - alpha q in v, xx = M^-1 s, y = A xx, (y, y) and (y, s) -> kStageOmega.
 // Grid nxb * ntj blocks (cooperative), block 32 * ceil(NZ / (2 NP)) threads.
+// An iteration (two of these and the update) against the separate launches: 20x20x30 47 us (63), 120x120x30 64
+// (88), 180x180x30 99 (143), 240x240x30 158 (216).  16 iterations in one launch, with both stages in one kernel,
+// spilled 600 to 1500 bytes a thread and took 98 us at 120x120x30.
 template <int R, int NP, int VM, bool BS>
 __global__ void __launch_bounds__(32 * kRsMaxWarps, 1) k_resident(const __grid_constant__ RsArgs A) {
   extern __shared__ double sh[];

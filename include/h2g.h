@@ -34,7 +34,7 @@ extern "C" {
 #define H2G_NONFINITE 3       /* NaN/Inf in an input array or in the iteration */
 #define H2G_BAD_ARG 4         /* rejected on the host before any launch */
 #define H2G_CUDA_ERROR 5      /* a CUDA runtime call failed */
-#define H2G_TIMEOUT 6         /* a bounded device wait ran out (the fused sweep's TMA waits) */
+#define H2G_TIMEOUT 6         /* a bounded device wait ran out (between the resident tiles, or for a TMA copy) */
 #define H2G_UNSUPPORTED 7     /* input outside what the library implements (message says what) */
 
 /* ---- precision ---------------------------------------------------------------------- */
@@ -264,8 +264,8 @@ int h2g_get_sweep(h2g_solver *h, int *fused, int *chunks, int *dd_array);
  * h2g_get_coop reports what the next solve uses.  No reference counterpart. */
 int h2g_set_coop(h2g_solver *h, int mode);
 int h2g_get_coop(h2g_solver *h, int *on);
-/* Budget of one bounded device wait (the fused sweep's waits for its TMA copies, the cooperative
- * preconditioner's grid barriers), in SM clock cycles; default about one second.  0 makes every
+/* Budget of one bounded device wait (the resident tiles' waits for one another, the fused sweep's for its
+ * TMA copies, the cooperative preconditioner's grid barriers), in SM clock cycles; default about one second.  0 makes every
  * such wait give up at once: the solve then ends with H2G_TIMEOUT, copies in flight are drained
  * and the context stays usable (the failure path of the bounded waits, exercised by the tests
  * without a GPU fault). */
