@@ -127,11 +127,11 @@ struct OpParams {
   const unsigned long long* nkey;  // per cell: own key and the 6 neighbours' keys, one byte each
   const uint16_t* cls; // per cell: stencil class (0xffff: not updated), may be null
   const T* ctab;       // [classes][8]: cxm, cxp, cym, cyp, czm, czp, dd, RN(1/dd) (FP64)
-  int cls_dd;          // the classes' dd is the cells' own (else a_p0 is missing from it: dd from ddv)
   T czm, czp;          // convective terms of the z-, z+ faces
   T dx0, dy0, ddt;
   int P;
   int steady;
+  int cls_dd;          // the classes' dd is the cells' own (else a_p0 is missing from it: dd from ddv)
 };
 
 }  // namespace h2g
