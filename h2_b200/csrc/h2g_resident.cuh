@@ -274,13 +274,17 @@ __device__ __forceinline__ unsigned rs_progress(const unsigned* prog) {
   return v;
 }
 // Waits until the two warps have finished n passes: their planes are then up to date, and nobody reads
-// what this warp's next pass overwrites.
+// what this warp's next pass overwrites.  Lanes may read different counts, so the warp votes: all of its
+// lanes go on, or give up, in the same turn.
+__device__ __forceinline__ bool rs_planes_ready(const unsigned* below, const unsigned* above, unsigned n) {
+  return __all_sync(kFull, rs_progress(below) >= n && rs_progress(above) >= n);
+}
 __device__ __forceinline__ bool rs_wait_planes(const unsigned* below, const unsigned* above, unsigned n,
                                                const RsArgs& A) {
-  if (rs_progress(below) >= n && rs_progress(above) >= n) return true;
+  if (rs_planes_ready(below, above, n)) return true;
   const long long t0 = clock64();
   for (unsigned turn = 1;; ++turn) {
-    if (rs_progress(below) >= n && rs_progress(above) >= n) return true;
+    if (rs_planes_ready(below, above, n)) return true;
     if ((turn & 63u) == 0 && rs_give_up(t0, A)) return false;
   }
 }
