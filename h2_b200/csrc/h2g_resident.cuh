@@ -338,8 +338,9 @@ __device__ __forceinline__ void rs_row(const RsAddr& a, unsigned tab, unsigned o
     }
   }
   if constexpr (!SOR) {
-    n0 = add(p0, sub(q0, p0));
-    n1 = add(p1, sub(q1, p1));
+    // a cell without a class stays 0 whatever lies in its b or beside it (zero times infinity is not 0)
+    n0 = cl & 0xffffu ? add(p0, sub(q0, p0)) : 0.0;
+    n1 = cl >> 16 ? add(p1, sub(q1, p1)) : 0.0;
     sts<D>(a.x, n0);
     sts<D + PL>(a.x, n1);
   } else {
@@ -382,8 +383,7 @@ __device__ __forceinline__ void rs_each(F& f) {
 // (false ends the pass).
 // b: from shared memory (BS: bs, row 0 of the colour, the lane's element), or from the vector itself (bv,
 // pitches row and plane), loaded two rows ahead of its use; f and l are those of the first and last row.
-// (A cell without a class may get anything finite for b: its row of the table, zeros with dd = 1 and y = 0,
-// makes it 0.)
+// (What a cell without a class gets for b does not matter: rs_row leaves it as it is.)
 template <int R, bool BS, bool SOR, typename Mid>
 __device__ __forceinline__ bool rs_rows(RsAddr a, unsigned tab, unsigned oa, unsigned bs, const double* bv, int row,
                                         int plane, double (&f)[2], double (&l)[2], RsCoef (&k)[2], unsigned& cur,
@@ -830,7 +830,8 @@ __global__ void __launch_bounds__(32 * kRsMaxWarps, 1) k_resident(const __grid_c
       if (VM != 0) load_u(r + 1);
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
-        if (VM != 0) rs_coef(tab, kp[(c * R + r) * 32], 16u, cur, cf);  // cxa: x+ (plane 0), x- (plane 1)
+        const unsigned cl = kp[(c * R + r) * 32];
+        if (VM != 0) rs_coef(tab, cl, 16u, cur, cf);  // cxa: x+ (plane 0), x- (plane 1)
 #pragma unroll
         for (int w = 0; w < 2; ++w) {
           const int o = c ^ 1, cw = c * 2 + w, ow = o * 2 + w;
@@ -843,9 +844,9 @@ __global__ void __launch_bounds__(32 * kRsMaxWarps, 1) k_resident(const __grid_c
             const double dn = w ? xc[o * 2] : x[o * CP - PL], up = w ? x[o * CP + 2 * PL] : xc[o * 2 + 1];
             // cxa multiplies x+ in the first plane and x- in the second
             const double pa = (e != (w != 0)) ? ot : xc[ow], pb = (e != (w != 0)) ? xc[ow] : ot;
-            // a cell without a class: 0 - 1 * 0
-            const double out =
+            const double ax =
                 sub(rs_sum(cf[w], cf[w].cxa, cf[w].cxb, pa, pb, on[ow], om[ow], up, dn), mul(cf[w].dd, xc[cw]));
+            const double out = (w ? cl >> 16 : cl & 0xffffu) ? ax : 0.0;
             if (in) {
               A.y[ci] = out;
               if (VM == 1) {

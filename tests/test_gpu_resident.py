@@ -234,3 +234,33 @@ def test_sor_boxes(oracle, grid):
     assert np.array_equal(out[0][1], out[1][1], equal_nan=True) and np.array_equal(out[0][2], out[1][2], equal_nan=True)
     s.close()
     ref.close()
+
+
+@pytest.mark.parametrize("n", [(41, 37, 30), (198, 181, 30), (200, 222, 30), (129, 147, 60), (126, 290, 60)],
+                         ids=lambda n: "x".join(map(str, n)))
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_preconditioner_reads_only_updated_cells(oracle, n, bad):
+    """Guards and masked cells of bb may hold anything, as in the separate passes, which never read them; and
+    what is not finite in an updated cell stays out of the masked ones."""
+    prob = mode3_model(oracle, n[0], n[1], n[2])
+    rng = np.random.default_rng(3)
+    masked = np.zeros(prob.shape, dtype=bool)
+    masked[1:-1, 1:-1, 1:-1] = rng.uniform(size=(n[0], n[1], n[2])) < 0.0005
+    prob.wk["mask"][masked] = 0.0
+    guards = np.ones(prob.shape, dtype=bool)
+    guards[1:-1, 1:-1, 1:-1] = False
+    clean = random_interior(prob.shape, 4)
+    clean[masked] = 0.0
+    dirty = clean.copy(order="F")
+    dirty[guards | masked] = bad
+    inside = clean.copy(order="F")
+    inside[n[0] // 2, n[1] // 2, n[2] // 2] = bad
+    s, ref = make_solver(prob), make_solver(prob)
+    ref.set_tuning(8, 2)
+    want = ref.preconditioner(clean, "gs")
+    assert np.isfinite(want).all()
+    assert np.array_equal(s.preconditioner(clean, "gs"), want)
+    assert np.array_equal(s.preconditioner(dirty, "gs"), want)
+    assert np.array_equal(s.preconditioner(inside, "gs"), ref.preconditioner(inside, "gs"), equal_nan=True)
+    s.close()
+    ref.close()
