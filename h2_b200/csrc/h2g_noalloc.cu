@@ -13,11 +13,12 @@
 // that loads this library holds it (512 KiB) until the process exits.  Consequences:
 //   * at most kNoAllocMaxRows = 65536 interior rows (NY * NZ) per call; larger grids are
 //     rejected with H2G_BAD_ARG before any launch;
-//   * all calls share the array and it keeps the last call's contents: the ticket counts round to zero
-//     in every call, and calls that overlap on the GPU (several host threads, or
-//     several streams) race on it -- serialise them;
+//   * all calls on a device share the array, the ticket (which each call counts round to zero) and the
+//     result's place in the host page below, so the library runs them one after the other: a call holds its
+//     device's lock from its launch until it has read the norm.  Work already in a call's stream must
+//     therefore not wait for something that another thread does only after its own call here;
 //   * the first call on a device looks up the array's device address (cudaGetSymbolAddress) with
-//     that device current.
+//     that device current, and the first call of the process pins one page of the library's own host memory.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -232,6 +233,7 @@ static __attribute__((aligned(4096))) volatile double g_result[512];
 static double* g_result_dev[64] = {nullptr};
 
 static std::mutex g_mu;
+static std::mutex g_call_mu[kMaxDevices];  // one call at a time on a device
 static double* g_scratch_ptr[kMaxDevices] = {nullptr};
 
 // Device addresses of the scratch array and of the result page on the current device (looked up once per
@@ -289,6 +291,7 @@ extern "C" int h2g_calcrk_noalloc(int MX, int MY, int MZ, const double* theta, c
   for (int f = 0; f < 6; ++f) a.HC[f] = HC[f];
   a.steady = is_steady ? 1 : 0;
   a.r = r;
+  std::lock_guard<std::mutex> one(g_call_mu[dev]);
   const unsigned blocks = (unsigned)(((MY - 2 + kRows - 1) / kRows) * (MZ - 2));
   k_calcrk_rows<<<blocks, kThreads, 0, st>>>(a, scratch, result ? result + dev : scratch + kResult);
   if (cudaGetLastError() != cudaSuccess) return H2G_CUDA_ERROR;

@@ -299,10 +299,13 @@ int h2g_bench_kernel(h2g_solver *h, int kind, int reps, int *launches);
  * r (device, MX*MY*MZ) gets the interior, guard cells are left untouched.  Nothing is allocated:
  * the reduction uses a 512 KiB device array inside the library that every GPU loading it keeps
  * until exit, so grids with more than 65536 interior rows (NY*NZ) are rejected (H2G_BAD_ARG).
- * Calls share that array: calls that overlap on the GPU race and must be serialised.  The first
- * call on a device looks up the array's address.  stream may be NULL (legacy default stream); the
- * call copies *res to the host and synchronises the stream before it returns, so it must not be
- * issued while that stream is capturing a CUDA graph. */
+ * Calls on one device share that array; the library runs them one after the other, whatever threads
+ * and streams they come from (so work already in a call's stream must not wait for something that
+ * another thread does only after its own call).  The first call on a device looks up the array's
+ * address; the first call of the process pins one page of the library's own host memory, through
+ * which the norm returns.  stream may be NULL (legacy default stream); the call sets *res on the host
+ * and synchronises the stream before it returns, so it must not be issued while that stream is
+ * capturing a CUDA graph. */
 int h2g_calcrk_noalloc(int MX, int MY, int MZ, const double *theta, const double *b, const double *lambda,
                        const double *mask, const double *rho, const double *cp, const double *ZC, const double *dZ,
                        double dx, double dy, double dt, const double *HC, int is_steady, double *r, double *res,

@@ -71,3 +71,66 @@ def test_calcrk_noalloc_rejects_oversized_grid():
     st = lib.h2g_calcrk_noalloc(10, 1002, 102, one, one, one, one, one, one, one, one, 1e-5, 1e-5, 1.0,
                                 HC.ctypes.data_as(C.POINTER(C.c_double)), 1, one, C.byref(res), None)
     assert st == L.H2G_BAD_ARG and res.value == -1.0
+
+
+class _Call:
+    """A problem's arrays on the device and its call; the handle's residual and norm to compare with."""
+
+    def __init__(self, prob, stream=None):
+        import torch
+        w = prob.wk
+        self.prob = prob
+        s = h2_b200.Solver(*prob.shape)
+        s.set_grid(prob.ZC, prob.dZ, prob.dx, prob.dy, prob.dt, prob.HC, prob.is_steady)
+        s.set_fields(w["lam"], w["mask"], *((None, None) if prob.is_steady else (w["rho"], w["cp"])))
+        s.set_rhs(w["b"])
+        s.set_theta(w["theta"])
+        self.r_ref, self.res_ref = s.calc_rk()
+        s.close()
+        self.d = [_dev(torch, w[n]) for n in ("theta", "b", "lam", "mask", "rho", "cp")]
+        self.z = [torch.from_numpy(a.copy()).cuda() for a in (prob.ZC, prob.dZ)]
+        self.r = torch.zeros_like(self.d[0])
+        self.HC = np.ascontiguousarray(prob.HC, dtype=np.float64)
+        self.stream = stream
+        torch.cuda.synchronize()
+
+    def __call__(self):
+        p = self.prob
+        res = C.c_double(0.0)
+        st = L.load().h2g_calcrk_noalloc(*p.shape, *(C.c_void_p(t.data_ptr()) for t in self.d + self.z), p.dx, p.dy,
+                                         p.dt, self.HC.ctypes.data_as(C.POINTER(C.c_double)), int(p.is_steady),
+                                         C.c_void_p(self.r.data_ptr()), C.byref(res),
+                                         C.c_void_p(self.stream.cuda_stream) if self.stream else None)
+        assert st == 0
+        return res.value
+
+    def residual(self):
+        return self.r.cpu().numpy().reshape(self.prob.shape, order="F")[1:-1, 1:-1, 1:-1]
+
+
+def test_calcrk_noalloc_calls_from_several_threads(oracle):
+    """Calls on grids with different numbers of blocks, from threads with a stream each and from threads that
+    share one: every call returns its own norm, and so do the calls after them."""
+    import threading
+
+    import torch
+    shared = torch.cuda.Stream()
+    sizes = [(41, 37, 30), (120, 90, 30), (24, 20, 30), (64, 130, 30)]
+    calls = [_Call(mode3_model(oracle, *n), stream)
+             for n, stream in zip(sizes, (shared, shared, torch.cuda.Stream(), None))]
+    alone = [c() for c in calls]
+    got = [[] for _ in calls]
+
+    def work(q):
+        for _ in range(100):
+            got[q].append(calls[q]())
+
+    ts = [threading.Thread(target=work, args=(q,)) for q in range(len(calls))]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    for q, c in enumerate(calls):
+        assert got[q] == [alone[q]] * 100
+        assert c() == alone[q] and abs(alone[q] - c.res_ref) <= 1e-13 * c.res_ref
+        assert np.array_equal(c.residual(), c.r_ref[1:-1, 1:-1, 1:-1])
