@@ -121,6 +121,14 @@ __device__ __forceinline__ void sts(unsigned a, double v) {
   asm volatile("st.shared.f64 [%0+%1], %2;" ::"r"(a), "n"(D), "d"(v));
 }
 
+// A value that this launch overwrites: an ordinary load (a read-only one may return old values), which the
+// compiler may move like a read-only one: the value is used up before its place is written.
+__device__ __forceinline__ double ld_once(const double* p) {
+  double v;
+  asm("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+
 // Coefficients of a cell.  cxa multiplies the x-neighbour at the cell's own position in an even row of
 // the tile, cxb the other one; in an odd row they change places.
 struct RsCoef {
@@ -645,8 +653,8 @@ __global__ void __launch_bounds__(32 * kRsMaxWarps, 1) k_resident(const __grid_c
           const int ci = where(pl0, r, cw >> 1, cw & 1);
           lc[cw] = __ldg(A.lcls + ci);
           if (VM != 0) lr[cw] = __ldg(A.r + ci);
-          if (VM != 0) lq[cw] = __ldg(A.q + ci);
-          if (VM != 2) lv[cw] = __ldg(A.v + ci);
+          if (VM != 0) lq[cw] = VM == 1 ? ld_once(A.q + ci) : __ldg(A.q + ci);
+          if (VM != 2) lv[cw] = ld_once(A.v + ci);
         }
       }
     };

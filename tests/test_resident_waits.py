@@ -43,3 +43,17 @@ def test_a_wait_ends_for_the_whole_warp(name, reads):
     text = without_votes(body(name))
     for word in reads:
         assert word + "(" not in text, (name, word)
+
+
+def test_no_read_only_load_of_a_vector_that_the_launch_writes():
+    """Read-only loads (ld.global.nc) may return old values of memory that the same launch writes.  k_resident
+    writes v in stages 1 and 2, q (as y) in stage 1, xx and the row sums; the SOR kernel writes xx."""
+    code = re.sub(r"//[^\n]*", "", SOURCE)
+    resident = code[code.index(" k_resident("):code.index(" k_resident_sor(") if " k_resident_sor(" in code else None]
+    for vector in ("A.v", "A.y", "A.xx", "A.rowsum", "A.partials"):
+        assert "__ldg(" + vector not in resident, vector
+    for m in re.finditer(r"__ldg\(A\.q\b", resident):
+        assert resident[:m.start()].rstrip().endswith("VM == 1 ? ld_once(A.q + ci) :")
+    sor = code[code.index("k_resident_sor("):]
+    for vector in ("A.xx", "A.rowsum", "A.partials"):
+        assert "__ldg(" + vector not in sor, vector
