@@ -18,6 +18,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <vector>
+
 namespace h2g {
 
 constexpr double kFloatMin = 1.0e-37;  // src/common.jl:12
@@ -133,5 +135,24 @@ struct OpParams {
   int steady;
   int cls_dd;          // the classes' dd is the cells' own (else a_p0 is missing from it: dd from ddv)
 };
+
+// Keys of the solves' graphs are made of the members of what was captured, one by one: the bytes between and
+// behind the members of a struct are indeterminate, and a key that held them would differ from call to call.
+// The lists below do not compile when a member is added to its struct and not to them.
+template <typename... M>
+inline void append_bytes(std::vector<unsigned char>& key, const M&... m) {
+  const auto one = [&](const void* p, size_t n) {
+    const unsigned char* c = static_cast<const unsigned char*>(p);
+    key.insert(key.end(), c, c + n);
+  };
+  (one(&m, sizeof m), ...);
+}
+template <typename T>
+inline void append_members(std::vector<unsigned char>& key, const OpParams<T>& op) {
+  const auto& [MX, MY, MZ, NX, NY, NZ, HP, HI, HN, plane, n] = op.g;
+  append_bytes(key, MX, MY, MZ, NX, NY, NZ, HP, HI, HN, plane, n);
+  const auto& [g, kp, tx, ty, tz, conv, rc, dzk, ddv, tq, nkey, cls, ctab, czm, czp, dx0, dy0, ddt, P, steady, cls_dd] = op;
+  append_bytes(key, kp, tx, ty, tz, conv, rc, dzk, ddv, tq, nkey, cls, ctab, czm, czp, dx0, dy0, ddt, P, steady, cls_dd);
+}
 
 }  // namespace h2g

@@ -1296,12 +1296,10 @@ static int launch_cg_body(Solver* s, cudaStream_t cs, const OpParams<T>& opA, co
 template <typename T, typename TP>
 static std::vector<unsigned char> signature(const OpParams<T>& opA, const OpParams<TP>& opM, int smoother,
                                             const void* x) {
-  std::vector<unsigned char> v(sizeof opA + sizeof opM + sizeof smoother + sizeof x);
-  unsigned char* d = v.data();
-  memcpy(d, &opA, sizeof opA);
-  memcpy(d + sizeof opA, &opM, sizeof opM);
-  memcpy(d + sizeof opA + sizeof opM, &smoother, sizeof smoother);
-  memcpy(d + sizeof opA + sizeof opM + sizeof smoother, &x, sizeof x);
+  std::vector<unsigned char> v;
+  append_members(v, opA);
+  append_members(v, opM);
+  append_bytes(v, smoother, x);
   return v;
 }
 
@@ -1360,10 +1358,8 @@ static int make_loop_graph(Solver* s, SolveGraph& G, Body body) {
 }
 
 static void sign_resident(const Solver* s, std::vector<unsigned char>& sig) {
-  const unsigned char* d = reinterpret_cast<const unsigned char*>(&s->rs);
-  sig.insert(sig.end(), d, d + sizeof s->rs);
-  d = reinterpret_cast<const unsigned char*>(&s->rs_box);
-  sig.insert(sig.end(), d, d + sizeof s->rs_box);
+  const auto& [R, np, nxb, ntj, ntab] = s->rs;
+  append_bytes(sig, R, np, nxb, ntj, ntab, s->rs_box);
 }
 
 template <typename T, typename TX, typename TP>
@@ -2012,9 +2008,9 @@ static int solve_sor(Solver* s, double omega, double tol, int maxItr, int verbos
          (int)kStageSorInit);
   CKL();
   SolveGraph& G = s->graphs[kGSor][resident ? (s->sm_share ? 3 : 2) : 0];
-  std::vector<unsigned char> sig(sizeof op + sizeof omega);
-  memcpy(sig.data(), &op, sizeof op);
-  memcpy(sig.data() + sizeof op, &omega, sizeof omega);
+  std::vector<unsigned char> sig;
+  append_members(sig, op);
+  append_bytes(sig, omega);
   if (resident) sign_resident(s, sig);
   if (!G.exec || G.sig != sig) {
     int berr = H2G_OK;
