@@ -468,6 +468,7 @@ static int sweep_status(Solver* s) {
     CK(cudaMemset(s->rs_rowsum, 0, s->rs_rowsum_cap));
     CK(cudaMemcpy(s->rs_ctl, &c, sizeof c, cudaMemcpyHostToDevice));
   }
+  CK(cudaStreamSynchronize(cudaStreamLegacy));  // a non-blocking stream does not wait for these by itself
   return fail(H2G_TIMEOUT, "a bounded wait of the RB-GS preconditioner ran out");
 }
 
@@ -594,34 +595,45 @@ static ResidentPlan resident_plan(const Solver* s) {
   return no;
 }
 
+// A device buffer of the handle, allocated and cleared on first use.  False: not enough memory (*p stays null).
+template <typename T>
+static bool have(Solver* s, T** p, size_t bytes) {
+  if (*p) return true;
+  if (cudaMalloc(p, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    *p = nullptr;
+    return false;
+  }
+  return cudaMemsetAsync(*p, 0, bytes, s->stream) == cudaSuccess;
+}
+
 // Buffers, the tiles' own class numbers and the shared-memory attributes for the split pl.  pl.R = 0 on
-// return: a tile has more classes than fit beside its x and b.
+// return: a tile has more classes than fit beside its x and b, or the device has no memory left for the
+// buffers (the separate passes need none of them).
 static int resident_prepare(Solver* s, ResidentPlan& pl) {
   const Geo& g = s->g;
-  // room for every split (a handle may run with all SMs in one call and a share of them in the next) and for
-  // the guards' rows of k_resident_sor
-  const size_t box =
-      sizeof(ulonglong2) * ((size_t)(s->num_sms + 2 * pl.nxb) * ((g.NZ + 1) & ~1) * 2 * kRsBox + kRsZero);
-  if (!s->rs_ctl) {
-    const size_t nb = (size_t)pl.nxb * ((g.NY + kBY - 1) / kBY) * g.NZ;
-    CK(cudaMalloc(&s->rs_box, box));
-    CK(cudaMemset(s->rs_box, 0, box));
-    s->rs_box_cap = box;
-    s->rs_rowsum_cap = sizeof(ulonglong2) * 2 * nb * 8;
-    CK(cudaMalloc(&s->rs_rowsum, s->rs_rowsum_cap));
-    CK(cudaMemset(s->rs_rowsum, 0, s->rs_rowsum_cap));
-    CK(cudaMalloc(&s->rs_lcls, sizeof(uint16_t) * (size_t)g.n));
-    CK(cudaMemset(s->rs_lcls, 0, sizeof(uint16_t) * (size_t)g.n));
-    CK(cudaMalloc(&s->rs_list, sizeof(uint16_t) * (size_t)s->num_sms * kRsMaxTab));
-    CK(cudaMalloc(&s->rs_count, sizeof(int) * (size_t)s->num_sms));
-    RsCtl* c = nullptr;
-    CK(cudaMalloc(&c, sizeof(RsCtl)));
+  // messages of every split of the grid (a handle may run with all SMs in one call, in fewer and larger tiles,
+  // and a share of them in the next) and the guards' rows of k_resident_sor
+  const int tiles = std::min(s->num_sms, pl.nxb * g.NY);
+  s->rs_box_cap = sizeof(ulonglong2) * ((size_t)(tiles + 2 * pl.nxb) * ((g.NZ + 1) & ~1) * 2 * kRsBox + kRsZero);
+  s->rs_rowsum_cap = sizeof(ulonglong2) * 2 * (size_t)pl.nxb * ((g.NY + kBY - 1) / kBY) * g.NZ * 8;
+  const bool fresh = !s->rs_ctl;
+  if (!have(s, &s->rs_box, s->rs_box_cap) || !have(s, &s->rs_rowsum, s->rs_rowsum_cap) ||
+      !have(s, &s->rs_lcls, sizeof(uint16_t) * (size_t)g.n) ||
+      !have(s, &s->rs_list, sizeof(uint16_t) * (size_t)tiles * kRsMaxTab) ||
+      !have(s, &s->rs_count, sizeof(int) * (size_t)tiles) || !have(s, &s->rs_ctl, sizeof(RsCtl))) {
+    // what there was of them goes back: others may need it more
+    cudaFree(s->rs_box); cudaFree(s->rs_rowsum); cudaFree(s->rs_lcls); cudaFree(s->rs_list); cudaFree(s->rs_count);
+    s->rs_box = s->rs_rowsum = nullptr;
+    s->rs_lcls = s->rs_list = nullptr;
+    s->rs_count = nullptr;
+    pl.R = 0;
+    return H2G_OK;
+  }
+  if (fresh) {
     const RsCtl init{1ull, 0u, 0u};
-    if (cudaMemcpy(c, &init, sizeof init, cudaMemcpyHostToDevice) != cudaSuccess) {
-      cudaFree(c);
-      return fail(H2G_CUDA_ERROR, "initialising the resident preconditioner failed");
-    }
-    s->rs_ctl = c;
+    CK(cudaMemcpyAsync(s->rs_ctl, &init, sizeof init, cudaMemcpyHostToDevice, s->stream));
+    CK(cudaStreamSynchronize(s->stream));
     s->rs_ntab = 0;
   }
   if (!s->rs_ntab || s->rs_rows != pl.R) {  // the classes were built anew, or another split

@@ -264,3 +264,52 @@ def test_preconditioner_reads_only_updated_cells(oracle, n, bad):
     assert np.array_equal(s.preconditioner(inside, "gs"), ref.preconditioner(inside, "gs"), equal_nan=True)
     s.close()
     ref.close()
+
+
+class _FilledDevice:
+    """Takes the device's free memory but for about `leave` bytes."""
+
+    def __init__(self, leave):
+        import torch
+        torch.cuda.empty_cache()
+        self.rt = ctypes.CDLL("libcudart.so.12")
+        self.held = []
+        for chunk in (1 << 30, 1 << 26, 1 << 21):
+            while torch.cuda.mem_get_info()[0] > leave + chunk:
+                p = ctypes.c_void_p()
+                if self.rt.cudaMalloc(ctypes.byref(p), ctypes.c_size_t(chunk)):
+                    self.rt.cudaGetLastError()
+                    break
+                self.held.append(p)
+
+    def release(self):
+        for p in self.held:
+            self.rt.cudaFree(p)
+        self.held = []
+
+
+def test_without_memory_for_the_buffers(oracle, monkeypatch):
+    """A device without room for the messages of the tiles: the solve takes the separate passes, again on the next
+    call, and the resident form once there is room."""
+    import torch
+    prob = mode3_model(oracle, 254, 296)
+    s = make_solver(prob)
+    s.snapshot()
+    monkeypatch.setenv("H2G_RB_COOP", "0")  # the separate passes: tuned and captured
+    st, ref = s.solve("pbicgstab", tol=1e-8, maxItr=8, smoother="gs")
+    th = s.get_theta()
+    monkeypatch.delenv("H2G_RB_COOP")
+    held = _FilledDevice(12 << 20)
+    free = torch.cuda.mem_get_info()[0]
+    for _ in range(2):
+        s.snapshot(restore=True)
+        st2, res = s.solve("pbicgstab", tol=1e-8, maxItr=8, smoother="gs")
+        assert (st2, res.itr, res.res) == (st, ref.itr, ref.res) and res.launches == ref.launches
+        assert np.array_equal(s.get_theta(), th)
+    assert free < 15 << 20 and torch.cuda.mem_get_info()[0] >= free - (2 << 20)  # no buffer is kept
+    held.release()
+    s.snapshot(restore=True)
+    st2, res = s.solve("pbicgstab", tol=1e-8, maxItr=8, smoother="gs")
+    assert (st2, res.itr, res.res) == (st, ref.itr, ref.res) and res.launches == launches_of(s, res.itr)
+    assert np.array_equal(s.get_theta(), th)
+    s.close()
