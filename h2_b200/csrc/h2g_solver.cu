@@ -49,8 +49,10 @@ static int fail(int code, const char* fmt, ...) {
 #define CK(call)                                                                                      \
   do {                                                                                                \
     cudaError_t e_ = (call);                                                                          \
-    if (e_ != cudaSuccess) return fail(H2G_CUDA_ERROR, "%s: %s (%s:%d)", #call, cudaGetErrorString(e_), \
-                                       __FILE__, __LINE__);                                           \
+    if (e_ != cudaSuccess) {                                                                          \
+      cudaGetLastError(); /* a failed allocation is reported once, not by the next launch too */      \
+      return fail(H2G_CUDA_ERROR, "%s: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, __LINE__); \
+    }                                                                                                 \
   } while (0)
 
 #define CKL()                                                                                             \
@@ -948,13 +950,10 @@ static int build_pairs(Solver* s, bool* ok) {
   const Geo& g = s->g;
   *ok = false;
   constexpr int kIds = 1 << 15;
-  if (!s->pair) {
-    CK(cudaMalloc(&s->pair, (size_t)g.n));
-    CK(cudaMalloc(&s->pair_num, kIds + 128));
-    CK(cudaMalloc(&s->pair_bits, kIds / 8));
-    CK(cudaMalloc(&s->pair_rc64, sizeof(double) * 128));
-    CK(cudaMalloc(&s->pair_rc32, sizeof(float) * 128));
-  }
+  // without memory for the pairs the classes hold no a_p0 either
+  if (!have(s, &s->pair, (size_t)g.n) || !have(s, &s->pair_num, kIds + 128) || !have(s, &s->pair_bits, kIds / 8) ||
+      !have(s, &s->pair_rc64, sizeof(double) * 128) || !have(s, &s->pair_rc32, sizeof(float) * 128))
+    return H2G_OK;
   const dim3 gi((g.NX + 255) / 256, g.NY, g.NZ);
   CK(cudaMemsetAsync(s->slots, 0xff, sizeof(unsigned long long) * kHashSlots, s->stream));
   CK(cudaMemsetAsync(s->flags, 0, sizeof(int), s->stream));
@@ -1017,15 +1016,13 @@ static int build_classes(Solver* s) {
     if (was) invalidate_graphs(s);
     return H2G_OK;
   }
-  if (!s->cls) {
-    CK(cudaMalloc(&s->cls, sizeof(uint16_t) * (size_t)g.n));
-    CK(cudaMalloc(&s->ctab, sizeof(double) * 8 * (size_t)kMaxClasses));
-    if (s->precision != H2G_FP64) CK(cudaMalloc(&s->ctab32, sizeof(float) * 8 * (size_t)kMaxClasses));
-    CK(cudaMalloc(&s->cslots, sizeof(unsigned long long) * kClassSlots));
-    CK(cudaMalloc(&s->slot_class, sizeof(uint16_t) * kClassSlots));
-    CK(cudaMalloc(&s->cwords, sizeof(unsigned long long) * kMaxClasses));
-    CK(cudaMalloc(&s->cflag, sizeof(int)));
-  }
+  if (!s->cls) CK(cudaMalloc(&s->cls, sizeof(uint16_t) * (size_t)g.n));
+  if (!s->ctab) CK(cudaMalloc(&s->ctab, sizeof(double) * 8 * (size_t)kMaxClasses));
+  if (!s->ctab32 && s->precision != H2G_FP64) CK(cudaMalloc(&s->ctab32, sizeof(float) * 8 * (size_t)kMaxClasses));
+  if (!s->cslots) CK(cudaMalloc(&s->cslots, sizeof(unsigned long long) * kClassSlots));
+  if (!s->slot_class) CK(cudaMalloc(&s->slot_class, sizeof(uint16_t) * kClassSlots));
+  if (!s->cwords) CK(cudaMalloc(&s->cwords, sizeof(unsigned long long) * kMaxClasses));
+  if (!s->cflag) CK(cudaMalloc(&s->cflag, sizeof(int)));
   bool pairs = false;
   if (!s->steady && s->rc64)
     if (int rc = build_pairs(s, &pairs)) return rc;

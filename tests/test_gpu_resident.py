@@ -313,3 +313,24 @@ def test_without_memory_for_the_buffers(oracle, monkeypatch):
     assert (st2, res.itr, res.res) == (st, ref.itr, ref.res) and res.launches == launches_of(s, res.itr)
     assert np.array_equal(s.get_theta(), th)
     s.close()
+
+
+def test_fields_on_a_full_device(oracle):
+    """h2g_set_fields of a transient grid on a device with little or no memory left either works, without what
+    there is no room for, or reports the failed allocation; once there is room the same handle works in full."""
+    prob = mode3_model(oracle, 200, 190, is_steady=False, dt=1e-4)
+    w = prob.wk
+    bb = random_interior(prob.shape, 2)
+    want = oracle.preconditioner(prob, bb, "gs")
+    for leave in (0, 2, 4, 8, 12, 16, 20, 24, 28, 36, 48, 64):
+        s = h2_b200.Solver(*prob.shape)
+        s.set_grid(prob.ZC, prob.dZ, prob.dx, prob.dy, prob.dt, prob.HC, False)
+        full = _FilledDevice(leave << 20)
+        try:
+            s.set_fields(w["lam"], w["mask"], w["rho"], w["cp"])
+        except h2_b200.H2GError as e:
+            assert e.status == L.H2G_CUDA_ERROR
+        full.release()
+        s.set_fields(w["lam"], w["mask"], w["rho"], w["cp"])
+        assert np.array_equal(s.preconditioner(bb, "gs"), want), leave
+        s.close()
