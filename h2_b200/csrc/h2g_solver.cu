@@ -564,18 +564,41 @@ class SmLease {
   int n_ = 0;
 };
 
+// What the resident form is asked for.
+enum class Resident { kPbicgstab, kCg, kSor };
+
+// Whether tiles of pl.R rows are faster than the separate passes.  A pass of the tiles takes as long with 5
+// planes as with 30 (the messages and waits of its rows), a separate pass takes as long as its cells, so tiles of
+// many rows need many planes.  The least number of planes by rows, with the ratio of an iteration's (a pass's) time
+// to the separate passes' there and below:
+//   PBiCGSTAB  3 rows  4: 0.92 (3: 1.05); 4 rows  8: 0.87 (5: 1.02); 5 to 8 rows 15: 0.94 - 0.99 (10: 1.07 - 1.20)
+//   CG         3 rows 10: 0.89 (5: 1.03); 4 rows on 17: 0.86 - 0.89 (15, 16: 0.99 - 1.05); its other kernels weigh more
+//   SOR        3 rows  4: 0.98 (3: 1.01); 4 rows  8: 0.95 (6: 1.03); 5 to 8 rows 12: 0.90 - 0.95 (8: 1.00 - 1.21)
+// Beyond 30 planes a warp has two pairs and a pass takes twice as long, so most of the SMs' positions must be in the
+// grid (70x70x60, half of them, 1 row: 97 -> 86 us an iteration; 145x145x60, 74 %: 200 -> 179; but 80x80x60, 34 %:
+// 103 -> 118, 100x100x60, 53 %: 116 -> 121), and the Krylov methods need more than 8 warps, 33 planes
+// (PBiCGSTAB 180x180: 32 planes 1.32, 33 1.01, 38 0.96; 145x145: 1.11, 0.94, 0.93; 240x148: 31 1.34, 34 0.93), CG
+// also no more than 2 rows (1 row 0.84, 2 rows 0.98, 3 and 4 rows 1.02 - 1.07).
+static bool resident_pays(const Geo& g, const ResidentPlan& pl, int sms, Resident what) {
+  static constexpr int kPlanes[3][kRsMaxRows + 1] = {
+      {0, 1, 1, 4, 8, 15, 15, 15, 15}, {0, 1, 1, 10, 17, 17, 17, 17, 17}, {0, 1, 1, 4, 8, 12, 12, 12, 12}};
+  if (pl.np == 1) return g.NZ >= kPlanes[(int)what][pl.R];
+  if (what != Resident::kSor && g.NZ < 33) return false;
+  if (what == Resident::kCg && pl.R > 2) return false;
+  return 100LL * g.NX * g.NY >= (pl.R == 1 ? 50LL : 65LL) * sms * 64 * pl.R;
+}
+
 // The split of k_resident for a grid, if it has one: tiles of 32 positions x R rows x all planes with
 // the fewest rows (the shortest pass) for which there is an SM for every tile; in a batch, first within
 // the handle's share of them.  A pass grows more slowly than its rows (its messages and barriers stay), so
 // two solves on halves beat two in turn on all: 120^2, 180^2 and 240^2 twice each, two threads, in turn 224 ms,
 // the first two on halves 192 ms (colour passes beside each other 218 ms).  A warp has one pair of
 // planes up to 30 planes (up to 8 rows: 240x240x30 takes 7, 140 tiles; 20x20 62.9 -> 47.4, 120x120 88 -> 64,
-// 240x240 216 -> 158 us an iteration), two pairs up to 60 planes (4 rows) if the grid fills the tiles: 70x70x60
-// (half of the positions, 1 row) 97 -> 86, 145x145x60 (74 %) 200 -> 179, but 80x80x60 (34 %) 103 -> 118, 100x100x60
-// (53 %) 116 -> 121.  Larger grids keep the separate launches, as do the grids without a class table or with tiles of
+// 240x240 216 -> 158 us an iteration), two pairs up to 60 planes (4 rows).  Larger grids keep the separate
+// launches, as do those that resident_pays leaves to them, the grids without a class table or with tiles of
 // too many classes (resident_prepare), the FP32 smoother, and handles on which a launch shape, a
 // coefficient source or another form of the preconditioner was asked for.
-static ResidentPlan resident_plan(const Solver* s) {
+static ResidentPlan resident_plan(const Solver* s, Resident what) {
   ResidentPlan no, pl;
   const Geo& g = s->g;
   if (s->precision != H2G_FP64 || !s->cls_ok || !s->recip_ok || !(s->steady || s->cls_rc) || s->nrhs) return no;
@@ -590,9 +613,8 @@ static ResidentPlan resident_plan(const Solver* s) {
     for (pl.R = 1; pl.R <= (pl.np == 1 ? kRsMaxRows : 4); ++pl.R) {
       pl.ntj = (g.NY + pl.R - 1) / pl.R;
       if (pl.blocks() > sms) continue;
-      // two pairs a warp: a pass takes twice as long, so most of the SMs' positions must be in the grid
-      if (pl.np == 2 && 100LL * g.NX * g.NY < (pl.R == 1 ? 50LL : 65LL) * sms * 64 * pl.R) break;
-      return pl;
+      if (resident_pays(g, pl, sms, what)) return pl;
+      break;
     }
   return no;
 }
@@ -1915,7 +1937,7 @@ struct ResidentCall {
   SmLease lease;
   // solveSOR!: the relaxation's quotient by its reciprocal needs omega within 2^+-100 (div_by)
   int begin_sor(Solver* solver, double omega) {
-    ResidentPlan pl = omega >= 0x1p-100 ? resident_plan(solver) : ResidentPlan();
+    ResidentPlan pl = omega >= 0x1p-100 ? resident_plan(solver, Resident::kSor) : ResidentPlan();
     if (pl.R)
       if (int rc = resident_prepare(solver, pl)) return rc;
     if (!pl.R) return H2G_OK;
@@ -1926,9 +1948,9 @@ struct ResidentCall {
     s->rs = pl;
     return H2G_OK;
   }
-  int begin(Solver* solver, int smoother) {
+  int begin(Solver* solver, int smoother, Resident what) {
     s = solver;
-    ResidentPlan pl = smoother == H2G_SMOOTHER_GS ? resident_plan(s) : ResidentPlan();
+    ResidentPlan pl = smoother == H2G_SMOOTHER_GS ? resident_plan(s, what) : ResidentPlan();
     if (pl.R)
       if (int rc = resident_prepare(s, pl)) return rc;
     if (pl.R) {
@@ -1958,7 +1980,7 @@ static int solve(Solver* s, bool cg, double tol, int maxItr, int smoother, int v
   if (!(tol >= 0.0) || !std::isfinite(tol)) return fail(H2G_BAD_ARG, "bad tolerance");
   CK(cudaSetDevice(s->device));
   ResidentCall resident;
-  if (int rc = resident.begin(s, smoother)) return rc;
+  if (int rc = resident.begin(s, smoother, cg ? Resident::kCg : Resident::kPbicgstab)) return rc;
   int rc;
   if (s->precision == H2G_MIXED_IR) rc = solve_ir(s, cg, tol, maxItr, smoother, verbose, res_hist, out);
   else if (s->precision == H2G_MIXED) rc = solve_mixed(s, cg, tol, maxItr, smoother, verbose, res_hist, out);
@@ -2904,7 +2926,7 @@ static int precond_t(Solver* s, const double* bb, double* xx, int smoother, cons
   void *ha, *hb;
   int rc;
   ResidentCall resident;  // before the hook buffers are filled: the tuner uses them
-  if ((rc = resident.begin(s, smoother))) return rc;
+  if ((rc = resident.begin(s, smoother, Resident::kPbicgstab))) return rc;
   if ((rc = hook_buffers(s, &ha, &hb))) return rc;
   T* xd = static_cast<T*>(ha);
   T* bd = static_cast<T*>(hb);
@@ -3193,7 +3215,9 @@ int h2g_batch_solve(int n, h2g_solver* const* hs, int method, double tol, int ma
   for (int q = 0; q < n; ++q) {
     const Solver* s = S(hs[q]);
     order[q] = q;
-    const h2g::ResidentPlan pl = method == 2 || smoother == H2G_SMOOTHER_GS ? h2g::resident_plan(s) : h2g::ResidentPlan();
+    const h2g::Resident what = method == 2 ? h2g::Resident::kSor : method == 1 ? h2g::Resident::kCg : h2g::Resident::kPbicgstab;
+    const h2g::ResidentPlan pl =
+        method == 2 || smoother == H2G_SMOOTHER_GS ? h2g::resident_plan(s, what) : h2g::ResidentPlan();
     if (pl.R && nt > 1) rank[q] = pl.blocks() > s->sm_share ? 0 : 1;
   }
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) {

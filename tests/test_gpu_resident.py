@@ -334,3 +334,41 @@ def test_fields_on_a_full_device(oracle):
         s.set_fields(w["lam"], w["mask"], w["rho"], w["cp"])
         assert np.array_equal(s.preconditioner(bb, "gs"), want), leave
         s.close()
+
+
+# grids of uniform layers: (NX, NY, NZ), then whether PBiCGSTAB, CG and SOR are resident
+ROUTES = [((240, 240, 14), (0, 0, 1)), ((240, 240, 15), (1, 0, 1)), ((240, 240, 17), (1, 1, 1)),
+          ((240, 240, 2), (0, 0, 0)), ((180, 180, 7), (0, 0, 0)), ((180, 180, 8), (1, 0, 1)),
+          ((90, 212, 3), (0, 0, 0)), ((90, 212, 4), (1, 0, 1)), ((90, 212, 10), (1, 1, 1)),
+          ((124, 140, 1), (1, 1, 1)), ((180, 180, 31), (0, 0, 1)), ((180, 180, 33), (1, 0, 1)),
+          ((120, 120, 32), (0, 0, 1)), ((120, 120, 35), (1, 1, 1)), ((70, 70, 33), (1, 1, 1)), ((60, 60, 45), (0, 0, 0)),
+          ((63, 148, 30), (1, 1, 1)), ((127, 120, 29), (1, 1, 1)), ((254, 290, 27), (1, 1, 1)),
+          ((127, 147, 57), (1, 0, 1))]
+
+
+@pytest.mark.parametrize("n,resident", ROUTES, ids=["x".join(map(str, r[0])) for r in ROUTES])
+def test_routes(oracle, n, resident):
+    """Both sides of the rule by rows and planes, odd numbers of planes beyond 30 and tiles along the positions whose
+    last one holds nothing but a guard: the route, and the separate passes' bits."""
+    prob = box_problem(oracle, *n, seed=1)
+    w = prob.wk
+    w["lam"][...] = np.array([0.4, 1.5, 50.0, 149.0])[np.arange(prob.shape[2]) // 2 % 4][None, None, :]
+    s, ref = make_solver(prob), make_solver(prob)
+    ref.set_tuning(8, 2)
+    bb = random_interior(prob.shape, 7)
+    assert np.array_equal(s.preconditioner(bb, "gs"), ref.preconditioner(bb, "gs"))
+    for method, route in zip(("pbicgstab", "cg", "sor"), resident):
+        got = []
+        for q in (s, ref):
+            q.set_theta(w["theta"])
+            hist = np.zeros(6)
+            if method == "sor":
+                st, res = q.sor(omega=1.2, tol=0.0, maxItr=6, hist=hist)
+            else:
+                st, res = q.solve(method, tol=0.0, maxItr=6, smoother="gs", hist=hist)
+            got.append((st, res.itr, hist, q.get_theta(), res.launches))
+        assert got[0][:2] == got[1][:2]
+        assert np.array_equal(got[0][2], got[1][2]) and np.array_equal(got[0][3], got[1][3])
+        assert (got[0][4] != got[1][4]) == bool(route), method
+    s.close()
+    ref.close()
