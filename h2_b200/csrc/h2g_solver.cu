@@ -1935,9 +1935,11 @@ static int autotune(Solver* s);
 struct ResidentCall {
   Solver* s = nullptr;
   SmLease lease;
-  // solveSOR!: the relaxation's quotient by its reciprocal needs omega within 2^+-100 (div_by)
-  int begin_sor(Solver* solver, double omega) {
-    ResidentPlan pl = omega >= 0x1p-100 ? resident_plan(solver, Resident::kSor) : ResidentPlan();
+  // solveSOR!: the relaxation's quotient by its reciprocal needs omega within 2^+-100 (div_by), and the tiles'
+  // set-up takes the time of one to two passes (a call of 1, 2 and 4 passes, us: 40x40x30 57, 67, 82, separate
+  // 44, 63, 93; 120x120x30 68, 78, 96, separate 56, 70, 106; 240x240x30 103, 121, 159, separate 85, 120, 185)
+  int begin_sor(Solver* solver, double omega, int maxItr) {
+    ResidentPlan pl = omega >= 0x1p-100 && maxItr > 2 ? resident_plan(solver, Resident::kSor) : ResidentPlan();
     if (pl.R)
       if (int rc = resident_prepare(solver, pl)) return rc;
     if (!pl.R) return H2G_OK;
@@ -2029,7 +2031,7 @@ static int solve_sor(Solver* s, double omega, double tol, int maxItr, int verbos
   int rc = ensure_hist(s, maxItr);
   if (rc) return rc;
   ResidentCall call;
-  if ((rc = call.begin_sor(s, omega))) return rc;
+  if ((rc = call.begin_sor(s, omega, maxItr))) return rc;
   const bool resident = s->rs.R != 0;
   const OpParams<double> op = op_params<double>(s, s->t64);
   SolverState* st = s->st;

@@ -372,3 +372,18 @@ def test_routes(oracle, n, resident):
         assert (got[0][4] != got[1][4]) == bool(route), method
     s.close()
     ref.close()
+
+
+@pytest.mark.parametrize("passes,resident", [(1, False), (2, False), (3, True), (33, True)])
+def test_sor_of_few_passes(oracle, passes, resident):
+    """A call of one or two passes does not pay for the tiles' set-up: it takes the separate passes."""
+    prob = mode3_model(oracle, 41, 37)
+    s, ref = make_solver(prob), make_solver(prob)
+    ref.set_tuning(8, 2)
+    got = [q.sor(omega=1.3, tol=0.0, maxItr=passes) + (q.get_theta(),) for q in (s, ref)]
+    assert got[0][0] == got[1][0] and got[0][1].res == got[1][1].res and got[0][1].itr == passes
+    assert np.array_equal(got[0][2], got[1][2])
+    assert got[1][1].launches == 2 + 2 * passes
+    assert got[0][1].launches == (2 + (passes + 31) // 32 if resident else 2 + 2 * passes)
+    s.close()
+    ref.close()
