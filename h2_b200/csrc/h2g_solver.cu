@@ -12,6 +12,7 @@
 #include <algorithm>
 #include <array>
 #include <atomic>
+#include <chrono>
 #include <map>
 #include <cmath>
 #include <condition_variable>
@@ -99,11 +100,23 @@ struct OpTables {
   int pcap = 0;
 };
 
-// How k_resident splits the grid: R rows and np pairs of planes of a warp, nxb x ntj tiles (R = 0: unused).
+// How k_resident splits the grid: R rows and np pairs of planes of a warp, nxb x ntj tiles (R = 0: unused), made to
+// run on a part of the SMs beside parts - 1 others.
 struct ResidentPlan {
-  int R = 0, np = 0, nxb = 0, ntj = 0, ntab = 0;
+  int R = 0, np = 0, nxb = 0, ntj = 0, ntab = 0, smem = 0, parts = 1;
   int blocks() const { return nxb * ntj; }
   int threads(int NZ) const { return 32 * ((NZ + 2 * np - 1) / (2 * np)); }
+};
+
+// The tiles' own class numbers for tiles of one number of rows: per cell, per tile its classes and how many;
+// rows of the largest tile's table (0: to be made), the shared memory of a block, and whether it has that much.
+struct ResidentTables {
+  uint16_t* lcls = nullptr;
+  uint16_t* list = nullptr;
+  int* count = nullptr;
+  int ntab = 0;
+  size_t smem = 0;
+  bool fits = false;
 };
 
 struct Solver {
@@ -163,7 +176,7 @@ struct Solver {
   size_t partials_cap = 0;
   double* hist = nullptr;
   int hist_cap = 0;
-  SolveGraph graphs[kGNum][4];  // smoother none, gs, gs with the resident preconditioner on all SMs, on a share
+  SolveGraph graphs[kGNum][2 + kRsMaxRows];  // smoother none, gs, gs with resident tiles of 1, 2, ... rows
   // mixed-precision refinement settings
   double inner_tol = 1e-4;
   int max_outer = 40;
@@ -214,7 +227,7 @@ struct Solver {
   double div_limit = 0.0;   // divergence stop of the next solves' states (mixed FP32 passes only)
   int coop_blocks = 0;      // blocks of the launch: SMs x resident blocks per SM
   bool coop_barred = false; // set while h2g_batch_solve runs the handle beside others
-  int sm_share = 0;         // SMs k_resident may take there (0: all)
+  int beside = 0;           // solves that it runs beside each other (0: no batch)
   GridBar* gbar = nullptr;
   long long wait_limit = kWaitCycles;  // budget of one bounded wait (clock cycles)
   std::map<std::pair<const void*, int>, CUtensorMap> xmaps;  // TMA maps of x buffers (pointer, bytes/element)
@@ -226,14 +239,9 @@ struct Solver {
   ulonglong2* rs_rowsum = nullptr;
   size_t rs_box_cap = 0, rs_rowsum_cap = 0;
   RsCtl* rs_ctl = nullptr;
-  uint16_t* rs_lcls = nullptr;  // per cell: class in its tile's numbering; per tile: its classes, their number
-  uint16_t* rs_list = nullptr;
-  int* rs_count = nullptr;
-  int rs_ntab = 0;              // rows of the largest tile table (0: to be made)
-  int rs_rows = 0;              // R of the split that the tables are for
-  size_t rs_smem = 0;
+  ResidentTables rs_tab[kRsMaxRows + 1];  // by rows of a tile
+  int rs_rows = 0;              // rows of the tiles whose messages the box holds
   int rs_most = 0;              // dynamic shared memory that the kernels may ask for
-  bool rs_fits = false;
   // K right-hand sides on the handle's operator (h2g_create_multi): stacked vectors, K states
   int nrhs = 0;
   double* mr_th = nullptr;
@@ -533,7 +541,18 @@ struct SmPool {
   std::condition_variable cv;
   int used = 0;
   unsigned long long next = 0, serving = 0;
+  struct Call {
+    unsigned long long stream;
+    bool legacy, blocking, over;
+    std::thread::id thread;
+    std::chrono::steady_clock::time_point end;
+  };
+  std::vector<Call> calls;  // in flight (that have their SMs or wait for them), and over for less than kBetween
 };
+// A thread that calls in a loop is between two calls for less than this: without it the threads of a loop find
+// each other missing now and then and change their splits (120x120x30, two threads: 60.8 us an iteration and
+// solve instead of 50.8).
+constexpr std::chrono::microseconds kBetween(1000);
 constexpr int kMaxDevices = 64;
 static SmPool g_sm_pool[kMaxDevices];
 
@@ -543,12 +562,52 @@ class SmLease {
   SmLease(const SmLease&) = delete;
   SmLease& operator=(const SmLease&) = delete;
   ~SmLease() {
-    if (!n_) return;
+    if (!pool_) return;
     std::lock_guard<std::mutex> lk(pool_->mu);
+    if (entered_)
+      for (SmPool::Call& c : pool_->calls)
+        if (!c.over && c.thread == me_.thread) {
+          c.over = true;
+          c.end = std::chrono::steady_clock::now();
+        }
+    if (!n_) return;
     pool_->used -= n_;
     pool_->cv.notify_all();
   }
-  void take(const Solver* s, int n) {
+  // Enters the call and returns how many streams of different threads have calls that can run beside each other, its
+  // own among them: calls on one stream take turns, and so do the legacy stream and the streams that wait for it.
+  int enter(const Solver* s) {
+    unsigned flags = 0;
+    if (cudaStreamGetId(s->stream, &me_.stream) != cudaSuccess || cudaStreamGetFlags(s->stream, &flags) != cudaSuccess) {
+      cudaGetLastError();
+      return 1;
+    }
+    me_.legacy = !s->stream || s->stream == cudaStreamLegacy;
+    me_.blocking = !me_.legacy && !(flags & cudaStreamNonBlocking);
+    me_.over = false;
+    me_.thread = std::this_thread::get_id();
+    pool_ = &g_sm_pool[s->device];
+    std::lock_guard<std::mutex> lk(pool_->mu);
+    auto& calls = pool_->calls;
+    const auto now = std::chrono::steady_clock::now();
+    calls.erase(std::remove_if(calls.begin(), calls.end(),
+                               [&](const SmPool::Call& c) {
+                                 return c.over && (c.thread == me_.thread || now - c.end > kBetween);
+                               }),
+                calls.end());
+    std::vector<unsigned long long> others;
+    for (const SmPool::Call& c : calls)
+      if (c.thread != me_.thread && c.stream != me_.stream && !(c.legacy && me_.blocking) &&
+          !(c.blocking && me_.legacy) && std::find(others.begin(), others.end(), c.stream) == others.end())
+        others.push_back(c.stream);
+    calls.push_back(me_);
+    entered_ = true;
+    return 1 + (int)others.size();
+  }
+  // Waits for the SMs.  What is in the call's stream already is waited for first: no call holds SMs while its
+  // stream waits for work that another caller may yet have to issue.
+  int take(const Solver* s, int n) {
+    CK(cudaStreamSynchronize(s->stream));
     pool_ = &g_sm_pool[s->device];
     std::unique_lock<std::mutex> lk(pool_->mu);
     const unsigned long long mine = pool_->next++;
@@ -557,10 +616,13 @@ class SmLease {
     pool_->used += n;
     n_ = n;
     pool_->cv.notify_all();
+    return H2G_OK;
   }
 
  private:
   SmPool* pool_ = nullptr;
+  SmPool::Call me_ = {};
+  bool entered_ = false;
   int n_ = 0;
 };
 
@@ -588,17 +650,36 @@ static bool resident_pays(const Geo& g, const ResidentPlan& pl, int sms, Residen
   return 100LL * g.NX * g.NY >= (pl.R == 1 ? 50LL : 65LL) * sms * 64 * pl.R;
 }
 
+// Whether `beside` solves are faster on pl.parts parts of the SMs than as separate passes beside each other, which
+// fill each other's gaps.  At least 4 at a time (or all of them) do; more than 4 do with tiles of up to 4 rows (40x40x30,
+// 8 threads: 12.5 us an iteration and solve, 18.8 on 4 parts and as separate passes; but 80x80x30, 7 parts of 8 rows
+// 26.5, separate 21.1, 4 parts 21.1).  Fewer, with the others waiting their turn, do where the tiles are at their best:
+// 24 to 30 planes (4 threads: 120x120x10 on 2 parts 38.9, separate 26.5; 160x160x30 on 2 parts 82, separate 102;
+// 240x240x30 in turn 163, separate 202); all in turn not for CG, whose other kernels then wait too (240x240x30,
+// 2 threads: 115, separate 101), nor for more than two calls of SOR (200x200x30, 4 threads: 27.4, separate 24.9).  With
+// two pairs of planes a warp the tiles must be nearly full (62x148x60 on 2 and 4 parts 66, 60, separate 77, 76; 120x120x45
+// on 2 parts, 57 % full, 88, separate 78), and CG gains nothing (62x148x60 1.04 - 1.08).
+static bool resident_beside(const Geo& g, const ResidentPlan& pl, int sms, Resident what, int beside) {
+  if (pl.np == 2)
+    return what != Resident::kCg && pl.parts >= std::min(beside, 4) &&
+           100LL * g.NX * g.NY * g.NZ >= 80LL * sms * 64 * pl.R * 60;
+  if (pl.parts > 4) return pl.R <= 4;
+  if (pl.parts >= std::min(beside, 4)) return true;
+  if (g.NZ < 24) return false;
+  return pl.parts > 1 || what == Resident::kPbicgstab || (what == Resident::kSor && beside == 2);
+}
+
 // The split of k_resident for a grid, if it has one: tiles of 32 positions x R rows x all planes with
-// the fewest rows (the shortest pass) for which there is an SM for every tile; in a batch, first within
-// the handle's share of them.  A pass grows more slowly than its rows (its messages and barriers stay), so
-// two solves on halves beat two in turn on all: 120^2, 180^2 and 240^2 twice each, two threads, in turn 224 ms,
-// the first two on halves 192 ms (colour passes beside each other 218 ms).  A warp has one pair of
+// the fewest rows (the shortest pass) for which there is an SM for every tile.  A warp has one pair of
 // planes up to 30 planes (up to 8 rows: 240x240x30 takes 7, 140 tiles; 20x20 62.9 -> 47.4, 120x120 88 -> 64,
 // 240x240 216 -> 158 us an iteration), two pairs up to 60 planes (4 rows).  Larger grids keep the separate
 // launches, as do those that resident_pays leaves to them, the grids without a class table or with tiles of
 // too many classes (resident_prepare), the FP32 smoother, and handles on which a launch shape, a
 // coefficient source or another form of the preconditioner was asked for.
-static ResidentPlan resident_plan(const Solver* s, Resident what) {
+// Of `beside` solves beside each other each gets a part of the SMs, as many parts as there are solves (at most 8, SOR
+// 4), or as the grid has a split for: a pass grows more slowly than its rows (its messages and waits stay), so two
+// solves on halves beat two in turn on all.
+static ResidentPlan resident_plan(const Solver* s, Resident what, int beside) {
   ResidentPlan no, pl;
   const Geo& g = s->g;
   if (s->precision != H2G_FP64 || !s->cls_ok || !s->recip_ok || !(s->steady || s->cls_rc) || s->nrhs) return no;
@@ -609,13 +690,17 @@ static ResidentPlan resident_plan(const Solver* s, Resident what) {
   pl.np = g.NZ <= 2 * kRsMaxWarps ? 1 : 2;
   if (g.NZ > 4 * kRsMaxWarps) return no;
   pl.nxb = (g.HN + 31) / 32;
-  for (int sms : {s->sm_share, s->num_sms})
+  if (what == Resident::kSor && beside > 4) return no;
+  for (pl.parts = std::min(beside, what == Resident::kSor ? 4 : 8); pl.parts > 0; --pl.parts) {
+    const int sms = s->num_sms / pl.parts;
     for (pl.R = 1; pl.R <= (pl.np == 1 ? kRsMaxRows : 4); ++pl.R) {
       pl.ntj = (g.NY + pl.R - 1) / pl.R;
       if (pl.blocks() > sms) continue;
-      if (resident_pays(g, pl, sms, what)) return pl;
-      break;
+      if (!resident_pays(g, pl, sms, what)) break;
+      if (beside > 1 && !resident_beside(g, pl, sms, what, beside)) break;
+      return pl;
     }
+  }
   return no;
 }
 
@@ -641,16 +726,22 @@ static int resident_prepare(Solver* s, ResidentPlan& pl) {
   const int tiles = std::min(s->num_sms, pl.nxb * g.NY);
   s->rs_box_cap = sizeof(ulonglong2) * ((size_t)(tiles + 2 * pl.nxb) * ((g.NZ + 1) & ~1) * 2 * kRsBox + kRsZero);
   s->rs_rowsum_cap = sizeof(ulonglong2) * 2 * (size_t)pl.nxb * ((g.NY + kBY - 1) / kBY) * g.NZ * 8;
-  const bool fresh = !s->rs_ctl;
+  ResidentTables& t = s->rs_tab[pl.R];
+  const bool fresh = !s->rs_ctl, made = t.count;
   if (!have(s, &s->rs_box, s->rs_box_cap) || !have(s, &s->rs_rowsum, s->rs_rowsum_cap) ||
-      !have(s, &s->rs_lcls, sizeof(uint16_t) * (size_t)g.n) ||
-      !have(s, &s->rs_list, sizeof(uint16_t) * (size_t)tiles * kRsMaxTab) ||
-      !have(s, &s->rs_count, sizeof(int) * (size_t)tiles) || !have(s, &s->rs_ctl, sizeof(RsCtl))) {
+      !have(s, &s->rs_ctl, sizeof(RsCtl)) || !have(s, &t.lcls, sizeof(uint16_t) * (size_t)g.n) ||
+      !have(s, &t.list, sizeof(uint16_t) * (size_t)pl.blocks() * kRsMaxTab) ||
+      !have(s, &t.count, sizeof(int) * (size_t)pl.blocks())) {
     // what there was of them goes back: others may need it more
-    cudaFree(s->rs_box); cudaFree(s->rs_rowsum); cudaFree(s->rs_lcls); cudaFree(s->rs_list); cudaFree(s->rs_count);
-    s->rs_box = s->rs_rowsum = nullptr;
-    s->rs_lcls = s->rs_list = nullptr;
-    s->rs_count = nullptr;
+    if (fresh) {
+      cudaFree(s->rs_box); cudaFree(s->rs_rowsum); cudaFree(s->rs_ctl);
+      s->rs_box = s->rs_rowsum = nullptr;
+      s->rs_ctl = nullptr;
+    }
+    if (!made) {
+      cudaFree(t.lcls); cudaFree(t.list); cudaFree(t.count);
+      t = ResidentTables();
+    }
     pl.R = 0;
     return H2G_OK;
   }
@@ -658,24 +749,27 @@ static int resident_prepare(Solver* s, ResidentPlan& pl) {
     const RsCtl init{1ull, 0u, 0u};
     CK(cudaMemcpyAsync(s->rs_ctl, &init, sizeof init, cudaMemcpyHostToDevice, s->stream));
     CK(cudaStreamSynchronize(s->stream));
-    s->rs_ntab = 0;
+  } else if (s->rs_rows != pl.R) {
+    // another split writes other slots: none keeps a number from before
+    CK(cudaMemsetAsync(s->rs_box, 0, s->rs_box_cap, s->stream));
+    CK(cudaMemsetAsync(s->rs_rowsum, 0, s->rs_rowsum_cap, s->stream));
   }
-  if (!s->rs_ntab || s->rs_rows != pl.R) {  // the classes were built anew, or another split
-    s->rs_ntab = 0;
-    s->rs_rows = pl.R;
+  s->rs_rows = pl.R;
+  if (!t.ntab) {  // the classes were built anew
     std::vector<int> count(pl.blocks());
-    CK(launch_tile_classes(s->stream, g, s->cls, s->rs_lcls, s->rs_list, s->rs_count, pl.R, pl.nxb, pl.ntj));
-    CK(cudaMemcpyAsync(count.data(), s->rs_count, sizeof(int) * count.size(), cudaMemcpyDeviceToHost, s->stream));
+    CK(launch_tile_classes(s->stream, g, s->cls, t.lcls, t.list, t.count, pl.R, pl.nxb, pl.ntj));
+    CK(cudaMemcpyAsync(count.data(), t.count, sizeof(int) * count.size(), cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
-    s->rs_ntab = 1 + *std::max_element(count.begin(), count.end());
-    s->rs_smem = rs_smem(pl.R, g.NZ, s->rs_ntab, resident_b_shared(pl));
+    t.ntab = 1 + *std::max_element(count.begin(), count.end());
+    t.smem = rs_smem(pl.R, g.NZ, t.ntab, resident_b_shared(pl));
     int most = 0;
     CK(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device));
-    s->rs_fits = s->rs_ntab <= kRsMaxTab && s->rs_smem + 512 <= (size_t)most;
+    t.fits = t.ntab <= kRsMaxTab && t.smem + 512 <= (size_t)most;
     s->rs_most = most - 512;
   }
-  pl.ntab = s->rs_ntab;
-  if (!s->rs_fits) pl.R = 0;
+  pl.ntab = t.ntab;
+  pl.smem = (int)t.smem;
+  if (!t.fits) pl.R = 0;
   return H2G_OK;
 }
 
@@ -689,9 +783,10 @@ static RsArgs resident_args(const Solver* s, const OpParams<double>& op, double*
   a.partials = s->partials;
   a.box = s->rs_box + kRsZero;
   a.ctl = s->rs_ctl;
-  a.lcls = s->rs_lcls;
-  a.list = s->rs_list;
-  a.count = s->rs_count;
+  const ResidentTables& t = s->rs_tab[s->rs.R];
+  a.lcls = t.lcls;
+  a.list = t.list;
+  a.count = t.count;
   a.ntab = s->rs.ntab;
   a.err = s->sweep_err;
   a.limit = s->wait_limit;
@@ -704,7 +799,7 @@ static int launch_tiles(Solver* s, cudaStream_t cs, const void* kernel, void** a
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(s->rs.blocks());
   cfg.blockDim = dim3(s->rs.threads(s->g.NZ));
-  cfg.dynamicSmemBytes = s->rs_smem;
+  cfg.dynamicSmemBytes = s->rs.smem;
   cfg.stream = cs;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeCooperative;
@@ -910,8 +1005,10 @@ static void destroy(Solver* s) {
   cudaFree(s->cls); cudaFree(s->ctab); cudaFree(s->ctab32); cudaFree(s->cslots); cudaFree(s->slot_class); cudaFree(s->cwords);
   cudaFree(s->pair); cudaFree(s->pair_num); cudaFree(s->pair_bits); cudaFree(s->pair_rc64); cudaFree(s->pair_rc32);
   cudaFree(s->cflag); cudaFree(s->key_prev); cudaFree(s->kdiff);
-  cudaFree(s->rs_box); cudaFree(s->rs_rowsum); cudaFree(s->rs_ctl); cudaFree(s->rs_lcls); cudaFree(s->rs_list);
-  cudaFree(s->rs_count);
+  cudaFree(s->rs_box); cudaFree(s->rs_rowsum); cudaFree(s->rs_ctl);
+  for (auto& t : s->rs_tab) {
+    cudaFree(t.lcls); cudaFree(t.list); cudaFree(t.count);
+  }
   s->mr_graph.reset();
   cudaFree(s->mr_th); cudaFree(s->mr_b); cudaFree(s->mr_st); cudaFree(s->mr_ctl); cudaFree(s->mr_partials);
   cudaFree(s->mr_flag);
@@ -1031,7 +1128,7 @@ static int build_classes(Solver* s) {
   const bool was = s->cls_ok;
   s->cls_ok = false;
   s->ncls = 0;
-  s->rs_ntab = 0;
+  for (auto& t : s->rs_tab) t.ntab = 0;
   s->cls_rc = false;
   const char* e = getenv("H2G_CLS");
   if ((e && atoi(e) == 0) || g.NZ > 255 || !s->nkey) {
@@ -1389,15 +1486,16 @@ static int make_loop_graph(Solver* s, SolveGraph& G, Body body) {
 }
 
 static void sign_resident(const Solver* s, std::vector<unsigned char>& sig) {
-  const auto& [R, np, nxb, ntj, ntab] = s->rs;
-  append_bytes(sig, R, np, nxb, ntj, ntab, s->rs_box);
+  const auto& [R, np, nxb, ntj, ntab, smem, parts] = s->rs;  // parts: not the launches' business
+  append_bytes(sig, R, np, nxb, ntj, ntab, smem, s->rs_box, s->rs_rowsum, s->rs_ctl, s->rs_tab[R].lcls,
+               s->rs_tab[R].list, s->rs_tab[R].count);
 }
 
 template <typename T, typename TX, typename TP>
 static int get_graph(Solver* s, int kind, int smoother, const OpParams<T>& op, const OpParams<TP>& opM, TX* x,
                      SolverState* st, SolveGraph** out) {
   const bool resident = std::is_same<T, double>::value && std::is_same<TP, double>::value && s->rs.R && smoother;
-  SolveGraph& G = s->graphs[kind][resident ? (s->sm_share ? 3 : 2) : smoother ? 1 : 0];
+  SolveGraph& G = s->graphs[kind][resident ? 1 + s->rs.R : smoother ? 1 : 0];
   std::vector<unsigned char> sig = signature(op, opM, smoother, (const void*)x);
   sig.push_back(use_coop(s) ? 1 : 0);
   if (resident) sign_resident(s, sig);
@@ -1935,37 +2033,45 @@ static int autotune(Solver* s);
 struct ResidentCall {
   Solver* s = nullptr;
   SmLease lease;
+  // The split for one call: within a part of the SMs where other calls are in flight beside it.
+  int plan(Resident what, ResidentPlan& pl) {
+    pl = resident_plan(s, what, 1);
+    if (!pl.R) return H2G_OK;
+    const int beside = lease.enter(s);
+    if (s->beside > 1 || beside > 1) pl = resident_plan(s, what, s->beside ? s->beside : beside);
+    return pl.R ? resident_prepare(s, pl) : H2G_OK;
+  }
   // solveSOR!: the relaxation's quotient by its reciprocal needs omega within 2^+-100 (div_by), and the tiles'
   // set-up takes the time of one to two passes (a call of 1, 2 and 4 passes, us: 40x40x30 57, 67, 82, separate
   // 44, 63, 93; 120x120x30 68, 78, 96, separate 56, 70, 106; 240x240x30 103, 121, 159, separate 85, 120, 185)
   int begin_sor(Solver* solver, double omega, int maxItr) {
-    ResidentPlan pl = omega >= 0x1p-100 && maxItr > 2 ? resident_plan(solver, Resident::kSor) : ResidentPlan();
-    if (pl.R)
-      if (int rc = resident_prepare(solver, pl)) return rc;
+    s = solver;
+    ResidentPlan pl;
+    if (omega >= 0x1p-100 && maxItr > 2)
+      if (int rc = plan(Resident::kSor, pl)) return rc;
     if (!pl.R) return H2G_OK;
     CK(cudaFuncSetAttribute(resident_sor_kernel(pl.R, pl.np), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            solver->rs_most));
-    s = solver;
-    lease.take(s, pl.blocks());
+                            s->rs_most));
+    if (int rc = lease.take(s, pl.blocks())) return rc;
     s->rs = pl;
     return H2G_OK;
   }
   int begin(Solver* solver, int smoother, Resident what) {
     s = solver;
-    ResidentPlan pl = smoother == H2G_SMOOTHER_GS ? resident_plan(s, what) : ResidentPlan();
-    if (pl.R)
-      if (int rc = resident_prepare(s, pl)) return rc;
+    ResidentPlan pl;
+    if (smoother == H2G_SMOOTHER_GS)
+      if (int rc = plan(what, pl)) return rc;
     if (pl.R) {
       for (int vm = 0; vm < 3; ++vm)
         CK(cudaFuncSetAttribute(resident_kernel(pl.R, pl.np, vm), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 s->rs_most));
       if (!s->rb_tuned) s->ax_cls = true;  // CG's CalcAX: the class table, untimed
-      lease.take(s, pl.blocks());
+      if (int rc = lease.take(s, pl.blocks())) return rc;
       s->rs = pl;
       return H2G_OK;
     }
     if (int rc = autotune(s)) return rc;
-    if (use_coop(s) && smoother == H2G_SMOOTHER_GS && s->device < kMaxDevices) lease.take(s, s->num_sms);
+    if (use_coop(s) && smoother == H2G_SMOOTHER_GS && s->device < kMaxDevices) return lease.take(s, s->num_sms);
     return H2G_OK;
   }
   ~ResidentCall() {
@@ -2040,7 +2146,7 @@ static int solve_sor(Solver* s, double omega, double tol, int maxItr, int verbos
   launch(s, k_res_sor, ag, blk, s->stream, op, (const double*)s->th, (const double*)s->b, omega, st, s->partials,
          (int)kStageSorInit);
   CKL();
-  SolveGraph& G = s->graphs[kGSor][resident ? (s->sm_share ? 3 : 2) : 0];
+  SolveGraph& G = s->graphs[kGSor][resident ? 1 + s->rs.R : 0];
   std::vector<unsigned char> sig;
   append_members(sig, op);
   append_bytes(sig, omega);
@@ -3209,22 +3315,23 @@ int h2g_batch_solve(int n, h2g_solver* const* hs, int method, double tol, int ma
   // passes
   for (int q = 0; q < n; ++q) {
     S(hs[q])->coop_barred = nt > 1;
-    S(hs[q])->sm_share = nt > 1 ? S(hs[q])->num_sms / nt : 0;
+    S(hs[q])->beside = nt;
   }
-  // members whose resident solve takes more than a share run one at a time: first, so that no share waits
-  // beside them; then the ones with a share, the longest first; then the others in the order given
-  std::vector<int> order(n), rank(n, 2);
+  // the members that need the most SMs first, so that no smaller part waits beside them, of those with equal parts
+  // the longest first; then the others in the order given
+  std::vector<int> order(n), parts(n, 0);
   for (int q = 0; q < n; ++q) {
     const Solver* s = S(hs[q]);
     order[q] = q;
     const h2g::Resident what = method == 2 ? h2g::Resident::kSor : method == 1 ? h2g::Resident::kCg : h2g::Resident::kPbicgstab;
-    const h2g::ResidentPlan pl =
-        method == 2 || smoother == H2G_SMOOTHER_GS ? h2g::resident_plan(s, what) : h2g::ResidentPlan();
-    if (pl.R && nt > 1) rank[q] = pl.blocks() > s->sm_share ? 0 : 1;
+    if (nt == 1 || (method != 2 && smoother != H2G_SMOOTHER_GS)) continue;
+    const h2g::ResidentPlan pl = h2g::resident_plan(s, what, nt);
+    if (pl.R) parts[q] = pl.parts;
   }
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
-    if (rank[a] != rank[b]) return rank[a] < rank[b];
-    return rank[a] == 1 && S(hs[a])->g.n > S(hs[b])->g.n;
+    if (!parts[a] || !parts[b]) return parts[a] > 0 && !parts[b];
+    if (parts[a] != parts[b]) return parts[a] < parts[b];
+    return S(hs[a])->g.n > S(hs[b])->g.n;
   });
   std::atomic<int> next(0);
   std::vector<std::string> errs(n);
@@ -3252,7 +3359,7 @@ int h2g_batch_solve(int n, h2g_solver* const* hs, int method, double tol, int ma
     cudaStreamSynchronize(own[q]);
     s->stream = saved[q];
     s->coop_barred = false;
-    s->sm_share = 0;
+    s->beside = 0;
     cudaStreamDestroy(own[q]);
   }
   int worst = H2G_OK;

@@ -156,8 +156,9 @@ int h2g_release_cached(void);
  * keeps its own grid, fields, θ and b (set beforehand), gets its own non-blocking stream for the
  * batch, and its whole solve (a CUDA graph looping on the device) is issued from one of
  * `threads` host threads (<= 0: 2), so the solves run concurrently on the GPU.  Members that can
- * keep their iterate on the chip get a share of the SMs each (all / threads) or, where that is too
- * few, all of them in turn; the order of the solves follows from that.  method 0
+ * keep their iterate on the chip get a part of the SMs each (up to 8 at a time), or all of them in
+ * turn, where that is faster than the separate passes of all of them beside each other; the order of
+ * the solves follows from that.  method 0
  * PBiCGSTAB, 1 CG, 2 RB-SOR with omega = 1.  outs[q] receives handle q's result (the same values
  * as a lone h2g_pbicgstab/h2g_cg on that handle: kernels are deterministic).  Returns H2G_OK
  * when every member converged, else the first non-OK member status (H2G_BAD_ARG /

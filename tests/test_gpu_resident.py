@@ -322,7 +322,7 @@ def test_fields_on_a_full_device(oracle):
     w = prob.wk
     bb = random_interior(prob.shape, 2)
     want = oracle.preconditioner(prob, bb, "gs")
-    for leave in (0, 2, 4, 8, 12, 16, 20, 24, 28, 36, 48, 64):
+    for leave in (0, 4, 10, 16, 24, 40):
         s = h2_b200.Solver(*prob.shape)
         s.set_grid(prob.ZC, prob.dZ, prob.dx, prob.dy, prob.dt, prob.HC, False)
         full = _FilledDevice(leave << 20)
@@ -387,3 +387,73 @@ def test_sor_of_few_passes(oracle, passes, resident):
     assert got[0][1].launches == (2 + (passes + 31) // 32 if resident else 2 + 2 * passes)
     s.close()
     ref.close()
+
+
+@pytest.mark.parametrize("method", [0, 1, 2], ids=["pbicgstab", "cg", "sor"])
+def test_batch_parts(oracle, method):
+    """Eight threads: parts of the SMs for up to 4 (CG 8) members at a time, all of them in turn, or the separate
+    passes where those are faster beside each other (SOR of more than 4, CG that needs all SMs).  Twice, so that
+    the splits of a handle alternate; always the lone call's bits."""
+    sizes = [(62, 63), (200, 222), (121, 117), (41, 37), (62, 63), (121, 117), (24, 20), (41, 37)]
+    hs = [make_solver(mode3_model(oracle, *n)) for n in sizes]
+    ptr = (ctypes.c_void_p * len(hs))(*[s.h.value for s in hs])
+    lone = []
+    for s in hs:
+        s.snapshot()
+        res = s.solve("cg" if method else "pbicgstab", tol=1e-8, maxItr=40)[1] if method < 2 else \
+            s.sor(tol=1e-8, maxItr=40)[1]
+        lone.append((res.itr, res.res, s.get_theta(), res.launches))
+    for _ in range(2):
+        for s in hs:
+            s.snapshot(restore=True)
+        outs = (L.Result * len(hs))()
+        L.load().h2g_batch_solve(len(hs), ptr, method, 1e-8, 40, 1, 8, outs)
+        for q, (o, s) in enumerate(zip(outs, hs)):
+            assert (o.itr, o.res) == lone[q][:2] and np.array_equal(s.get_theta(), lone[q][2])
+            separate = method == 2 or (method == 1 and sizes[q] == (200, 222))
+            assert (o.launches != lone[q][3]) == separate
+    for s in hs:
+        s.close()
+
+
+def test_threads_on_parts(oracle):
+    """Host threads on streams of their own get parts of the SMs, threads that share the default stream take all of
+    them in turn; a thread's split changes with what is in flight.  Each call gives its lone call's bits."""
+    import torch
+    sizes = [(62, 63), (41, 37), (121, 117), (62, 63), (24, 20), (121, 117)]
+    probs = [mode3_model(oracle, *n) for n in sizes]
+    lone, got = [], [[] for _ in sizes]
+
+    def call(s):
+        s.snapshot(restore=True)
+        st, res = s.solve("pbicgstab", tol=1e-8, maxItr=50, smoother="gs")
+        out = (st, res.itr, res.res)
+        th = s.get_theta()
+        st, res = s.sor(tol=0.0, maxItr=20)
+        return out + (res.res, th, s.get_theta())
+
+    for p in probs:
+        s = make_solver(p)
+        s.snapshot()
+        lone.append(call(s))
+        s.close()
+
+    def work(q):
+        s = make_solver(probs[q])
+        if q < 4:
+            stream = torch.cuda.Stream()
+            L.check(s.lib.h2g_set_stream(s.h, ctypes.c_void_p(stream.cuda_stream)))
+        s.snapshot()
+        for _ in range(6):
+            got[q].append(call(s))
+        s.close()
+
+    ts = [threading.Thread(target=work, args=(q,)) for q in range(len(sizes))]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    for ref, out in zip(lone, got):
+        assert len(out) == 6
+        for g in out:
+            assert g[:4] == ref[:4] and np.array_equal(g[4], ref[4]) and np.array_equal(g[5], ref[5])
