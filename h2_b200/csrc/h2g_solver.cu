@@ -206,6 +206,7 @@ struct Solver {
   int* cflag = nullptr;
   // transient grids: (key, rho*cp) pairs in the classes (cls_rc), per cell and their keys and rho*cp
   bool cls_rc = false;
+  bool pairs_known = false, pairs_ok = false;  // build_pairs' last answer is that of the fields in place
   uint8_t* pair = nullptr;
   uint8_t* pair_num = nullptr;  // 2^15 pair numbers, then the pairs' keys (128)
   unsigned* pair_bits = nullptr;
@@ -1067,6 +1068,10 @@ static void invalidate_graphs(Solver* s) {
 // kMaxKeys pairs.
 static int build_pairs(Solver* s, bool* ok) {
   const Geo& g = s->g;
+  if (s->pairs_known) {  // another time step or Z grid: the pairs depend on the fields alone
+    *ok = s->pairs_ok;
+    return H2G_OK;
+  }
   *ok = false;
   constexpr int kIds = 1 << 15;
   // without memory for the pairs the classes hold no a_p0 either
@@ -1084,6 +1089,8 @@ static int build_pairs(Solver* s, bool* ok) {
   CK(cudaMemcpyAsync(slots.data(), s->slots, sizeof(unsigned long long) * kHashSlots, cudaMemcpyDeviceToHost, s->stream));
   CK(cudaMemcpyAsync(&flags, s->flags, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));
+  s->pairs_ok = false;
+  s->pairs_known = true;  // too many values or pairs, unless they turn out to fit
   if (flags) return H2G_OK;
   std::vector<int> index(kHashSlots, 0);
   std::vector<double> value;
@@ -1119,7 +1126,7 @@ static int build_pairs(Solver* s, bool* ok) {
   k_write_pairs<<<gi, 256, 0, s->stream>>>(g, s->key, s->rc64, s->slots, s->slot_index, s->pair_num, s->pair);
   CKL();
   CK(cudaStreamSynchronize(s->stream));  // the host vectors must outlive the copies
-  *ok = n > 0;
+  *ok = s->pairs_ok = n > 0;
   return H2G_OK;
 }
 
@@ -2882,6 +2889,7 @@ static int set_fields(Solver* s, const double* lam, const double* mask, const do
   if ((rho == nullptr) != (cp == nullptr)) return fail(H2G_BAD_ARG, "rho and cp must both be given or both be NULL");
   if (s->grid_set && !s->steady && !rho) return fail(H2G_BAD_ARG, "transient grid needs rho and cp");
   const Geo& g = s->g;
+  s->pairs_known = false;
   const size_t nf = sizeof(double) * (size_t)s->nfort();
   CK(cudaMemcpyAsync(s->stage[0], lam, nf, cudaMemcpyHostToDevice, s->stream));
   CK(cudaMemcpyAsync(s->stage[1], mask, nf, cudaMemcpyHostToDevice, s->stream));

@@ -457,3 +457,28 @@ def test_threads_on_parts(oracle):
         assert len(out) == 6
         for g in out:
             assert g[:4] == ref[:4] and np.array_equal(g[4], ref[4]) and np.array_equal(g[5], ref[5])
+
+
+def test_transient_grid_with_another_step(oracle):
+    """h2g_set_grid with another time step keeps the (key, rho cp) pairs of the fields and makes the classes anew;
+    h2g_set_fields finds the pairs again, too many of them included."""
+    prob = mode3_model(oracle, 41, 37, is_steady=False, dt=1e-4)
+    w = prob.wk
+    s = make_solver(prob)
+    bb = random_interior(prob.shape, 9)
+    rng = np.random.default_rng(4)
+    for scale, many, resident in ((1.0, False, True), (1.7, False, True), (1.7, True, False), (0.6, False, True)):
+        w["rho"][1:-1, 1:-1, 1:-1] *= scale * (1.0 + 0.01 * rng.integers(0, 40, (41, 37, 30)) if many else scale)
+        if not many:
+            w["rho"][...] = np.round(w["rho"], -2) + 100.0
+            w["cp"][...] = np.round(w["cp"], -3) + 1000.0
+            w["rho"][1:-1, 1:-1, 1:-1] = np.where(w["lam"][1:-1, 1:-1, 1:-1] > 1.0, 8000.0 * scale, 2000.0)
+        s.set_fields(w["lam"], w["mask"], w["rho"], w["cp"])
+        for dt in (1e-4, 3e-5, 2e-3):
+            prob.dt = dt
+            s.set_grid(prob.ZC, prob.dZ, prob.dx, prob.dy, dt, prob.HC, False)
+            assert np.array_equal(s.preconditioner(bb, "gs"), oracle.preconditioner(prob, bb, "gs")), (scale, many, dt)
+            s.set_theta(w["theta"])
+            st, res = s.solve("pbicgstab", tol=0.0, maxItr=3, smoother="gs")
+            assert (res.launches == launches_of(s, res.itr)) == resident
+    s.close()
