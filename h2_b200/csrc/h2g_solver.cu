@@ -2195,7 +2195,9 @@ static int solve_sor(Solver* s, double omega, double tol, int maxItr, int verbos
     out->res = fin.res;
   }
   if (resident) {
-    if (const int e = sweep_status(s)) {  // a bounded wait ran out: theta is that of the last whole launch
+    // A bounded wait ran out.  theta may be of no one pass: where only the wait for the end of a pass did, the blocks
+    // that saw it have written their tiles back and the one that gave up has not.
+    if (const int e = sweep_status(s)) {
       if (out) {
         out->status = e;
         out->isconverged = 0;

@@ -242,26 +242,30 @@ class Solver:
         return r.value, p.value, a.value, b.value
 
     def set_tuning(self, rows: int, planes: int = 2):
-        """Force the colour pass's shape (rows 2, 4, 8, 16; planes 1, 2); rows = 0 tunes again."""
+        """Force the colour pass's shape (rows 2, 4, 8, 16; planes 1, 2), and with it the separate passes instead
+        of the resident form; rows = 0 tunes again and allows the resident form again."""
         L.check(self.lib.h2g_set_tuning(self.h, int(rows), int(planes)))
 
     def set_sweep(self, fused: int, chunks: int = 1, dd_array: bool = False):
         """Force the preconditioner's sweeps 2-5: fused=1 one fused launch per sweep (with `chunks`
-        z chunks and dd read or summed), 0 two colour passes per sweep, -1 let the tuner choose."""
+        z chunks and dd read or summed), 0 two colour passes per sweep, -1 let the tuner choose.  0 and 1 also turn
+        the resident form off."""
         L.check(self.lib.h2g_set_sweep(self.h, int(fused), int(chunks), int(bool(dd_array))))
 
     def sweep(self) -> tuple:
-        """(fused, chunks, dd read) that the next solve uses (running the tuner if needed)."""
+        """(fused, chunks, dd read) that the next solve uses if it runs as separate passes (running the tuner if
+        needed)."""
         f, c, d = C.c_int(0), C.c_int(0), C.c_int(0)
         L.check(self.lib.h2g_get_sweep(self.h, C.byref(f), C.byref(c), C.byref(d)))
         return bool(f.value), c.value, bool(d.value)
 
     def set_coop(self, mode: int):
-        """The PBiCGSTAB preconditioner as one cooperative launch: 1 on, 0 off, -1 default."""
+        """The PBiCGSTAB preconditioner of the separate passes as one cooperative launch: 1 on, 0 no cooperative
+        launch of any kind (nor the resident form), -1 default."""
         L.check(self.lib.h2g_set_coop(self.h, int(mode)))
 
     def coop(self) -> bool:
-        """Whether the next solve runs the cooperative preconditioner."""
+        """Whether the next solve, if it runs as separate passes, uses the cooperative preconditioner."""
         on = C.c_int(0)
         L.check(self.lib.h2g_get_coop(self.h, C.byref(on)))
         return bool(on.value)

@@ -228,9 +228,25 @@ int h2g_calrhs(h2g_solver *h, const h2g_bc *bc, int zero_b);
 int h2g_transient(h2g_solver *h, const h2g_bc *bc, int nt, int method, double tol, int maxItr, int smoother,
                   int verbose, double *step_stats, h2g_result *out);
 
-/* ---- launch-shape tuning (no reference counterpart) ---------------------------------------
+/* ---- the form of a solve (no reference counterpart) ----------------------------------------
+ * FP64 solves and h2g_preconditioner with the RB-GS smoother, and h2g_sor calls of more than two
+ * passes, keep their iterate in the SMs' shared memory (k_resident, k_resident_sor) on grids of up to
+ * 60 planes that have an SM for every tile and for which that is the faster form; all others run as
+ * separate passes.  The results are the same bits.  The form shows in h2g_result.launches: 3 an
+ * iteration of PBiCGSTAB, 5 of CG, 1 for 32 passes of SOR, against 23, 14 and 2 a pass.
+ *
+ * The resident form is cooperative launches, which the GPU starts when it has SMs for all of their
+ * tiles: a solve waits for kernels of other streams that hold SMs, however long those run.  Where
+ * such a kernel itself waits for the result of the solve, turn the form off with h2g_set_coop(h, 0).
+ *
+ * Every request for a variant of the separate passes also turns the resident form off, until it is
+ * taken back: h2g_set_tuning (back: rows = 0), h2g_set_sweep and h2g_set_coop with mode 0 or 1 (back:
+ * -1), and H2G_RB_ROWS, H2G_RB_PLANES, H2G_RB_DD, H2G_AX_DD, H2G_RB_FUSED, H2G_SW_CHUNKS, H2G_SW_DD
+ * or H2G_RB_COOP in the environment, whatever their values; so does H2G_CLS=0.
+ *
+ * ---- launch-shape tuning of the separate passes (no reference counterpart) -------------------
  * The smoother's colour pass has no reduction, so its launch variant changes no result.  The
- * first solve of a handle times blocks of 2, 4, 8 and 16 rows with 1 or 2 planes per thread and
+ * first solve of a handle that runs as separate passes times blocks of 2, 4, 8 and 16 rows with 1 or 2 planes per thread and
  * three sources of a cell's coefficients (a few sweeps each on scratch vectors) and keeps the
  * fastest; it also times the FP64 CalcAX with each source (the same bits in every case).  The
  * sources: 0 the key tables with dd summed per cell, 1 the key tables with dd read from a
@@ -252,24 +268,27 @@ int h2g_set_tuning(h2g_solver *h, int rows, int planes);
  * faster (H2G_RB_FUSED, H2G_SW_CHUNKS, H2G_SW_DD in the environment force it).  h2g_set_sweep forces
  * the choice on a handle: fused 0 (colour passes), 1 (fused, with `chunks` z chunks, 1..255, and
  * dd read from the per-cell array if dd_array) or -1 (tune again); h2g_get_sweep reports what the
- * next solve uses.  No reference counterpart (rbsor!, NonUniform.jl:936-957, runs the colours one
+ * next solve uses if it runs as separate passes.  No reference counterpart (rbsor!, NonUniform.jl:936-957, runs the colours one
  * after another over the whole grid). */
 int h2g_set_sweep(h2g_solver *h, int fused, int chunks, int dd_array);
 int h2g_get_sweep(h2g_solver *h, int *fused, int *chunks, int *dd_array);
 /* The whole preconditioner of a PBiCGSTAB iteration (first pass and 9 colour passes) as one
  * cooperative launch with a bounded grid barrier between passes (k_precond_coop), instead of ten
- * launches; results bit-identical.  FP64 handles on the colour-pass path only.  mode 1 on, 0 off,
- * -1 default (off unless H2G_RB_COOP=1 in the environment).  h2g_batch_solve runs its handles
+ * launches; results bit-identical.  FP64 handles on the colour-pass path only.  mode 1 on, 0 no
+ * cooperative launch of any kind, -1 default (off unless H2G_RB_COOP=1 in the environment; the resident
+ * form where the grid has one).  h2g_batch_solve runs its handles
  * without it while more than one solve is in flight (a cooperative launch needs the device to
  * itself; beside another cooperative launch a barrier would wait until its budget ran out).
- * h2g_get_coop reports what the next solve uses.  No reference counterpart. */
+ * h2g_get_coop reports whether the next solve uses it if it runs as separate passes.  No reference
+ * counterpart. */
 int h2g_set_coop(h2g_solver *h, int mode);
 int h2g_get_coop(h2g_solver *h, int *on);
 /* Budget of one bounded device wait (the resident tiles' waits for one another, the fused sweep's for its
  * TMA copies, the cooperative preconditioner's grid barriers), in SM clock cycles; default about one second.  0 makes every
  * such wait give up at once: the solve then ends with H2G_TIMEOUT, copies in flight are drained
  * and the context stays usable (the failure path of the bounded waits, exercised by the tests
- * without a GPU fault). */
+ * without a GPU fault).  theta is then somewhere between its start and the solution, after h2g_sor not
+ * even the field of one pass: set it anew. */
 int h2g_set_wait_limit(h2g_solver *h, long long cycles);
 
 /* ---- kernels of the path, callable one at a time (host arrays in and out) ---------------

@@ -482,3 +482,38 @@ def test_transient_grid_with_another_step(oracle):
             st, res = s.solve("pbicgstab", tol=0.0, maxItr=3, smoother="gs")
             assert (res.launches == launches_of(s, res.itr)) == resident
     s.close()
+
+
+def test_switches(oracle, monkeypatch):
+    """What turns the resident form off, and back: the calls and the variables that ask for a variant of the
+    separate passes, as include/h2g.h lists them."""
+    prob = mode3_model(oracle, 41, 37)
+    s = make_solver(prob)
+    s.snapshot()
+
+    def forms():
+        out = []
+        for method, launches in (("pbicgstab", 2 + 3 * 5), ("sor", 2 + 1)):
+            s.snapshot(restore=True)
+            res = s.sor(tol=0.0, maxItr=5)[1] if method == "sor" else s.solve(method, tol=0.0, maxItr=5)[1]
+            out.append(res.launches == launches)
+        assert out[0] == out[1]
+        return out[0]
+
+    assert forms()
+    for off, back in ((lambda: s.set_tuning(8, 2), lambda: s.set_tuning(0)),
+                      (lambda: s.set_sweep(0), lambda: s.set_sweep(-1)),
+                      (lambda: s.set_sweep(1, 2), lambda: s.set_sweep(-1)),
+                      (lambda: s.set_coop(0), lambda: s.set_coop(-1)), (lambda: s.set_coop(1), lambda: s.set_coop(-1))):
+        off()
+        assert not forms()
+        back()
+        assert forms()
+    for name in ("H2G_RB_ROWS", "H2G_RB_PLANES", "H2G_RB_DD", "H2G_AX_DD", "H2G_RB_FUSED", "H2G_SW_CHUNKS", "H2G_SW_DD",
+                 "H2G_RB_COOP"):
+        monkeypatch.setenv(name, "0")
+        assert not forms(), name
+        monkeypatch.delenv(name)
+    s.autotune(), s.sweep(), s.coop()  # asking turns nothing off
+    assert forms()
+    s.close()
