@@ -146,3 +146,71 @@ def test_row_sums_have_one_owner(NY, R):
         if group * 8 < tj * R + R and group * 8 < NY:
             owners.setdefault(group, []).append(tj)
     assert sorted(owners) == list(range(-(-NY // 8))) and all(len(v) == 1 for v in owners.values())
+
+
+LAYOUT = r"""
+#include <cstdio>
+#include "h2g_resident.cuh"
+using namespace h2g;
+int main() {
+  printf("%d %d %d %d %d\n", kRsRowPitch, kRsBox, kRsTabRow, kRsMaxTab, kRsMaxWarps);
+  for (int R = 1; R <= kRsMaxRows; ++R)
+    for (int NZ = 1; NZ <= 4 * kRsMaxWarps; ++NZ)
+      for (int bs = 0; bs < 2; ++bs)
+        printf("%d %d %d %zu %zu\n", R, NZ, bs, rs_x_elems(R, NZ), rs_smem(R, NZ, 1, bs));
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def layout(tmp_path_factory):
+    """The kernel's own sizes: constants, elements of x, bytes of a block with a table of one row."""
+    import os
+    import subprocess
+
+    from conftest import ROOT
+    from h2_b200 import build
+    try:
+        nvcc = build.nvcc()
+    except RuntimeError:
+        pytest.skip("no nvcc")
+    d = tmp_path_factory.mktemp("layout")
+    (d / "layout.cu").write_text(LAYOUT)
+    subprocess.run([nvcc, "-std=c++17", "-O0", *build.ARCH, "-I", os.path.join(ROOT, "h2_b200", "csrc"),
+                    str(d / "layout.cu"), "-o", str(d / "layout")], check=True, capture_output=True)
+    out = subprocess.run([str(d / "layout")], check=True, capture_output=True, text=True).stdout.splitlines()
+    consts = dict(zip(("pitch", "box", "row", "most", "warps"), map(int, out[0].split())))
+    sizes = {tuple(v[:3]): tuple(v[3:]) for v in (list(map(int, line.split())) for line in out[1:])}
+    return consts, sizes
+
+
+@pytest.mark.parametrize("NZ", [1, 2, 9, 29, 30, 31, 32, 59, 60])
+def test_shared_memory_layout(layout, NZ):
+    """x, the table of the tile's classes, b and the classes lie one behind the other inside the block's shared memory,
+    for every split; the neighbours of every cell lie inside x, the planes of zeros around it included."""
+    consts, sizes = layout
+    assert consts["pitch"] == 34 and consts["box"] == BOX
+    np_ = 1 if NZ <= 30 else 2
+    for R in range(1, (8 if np_ == 1 else 4) + 1):
+        bs = b_shared(R, np_)
+        x, one = sizes[R, NZ, int(bs)]
+        P, PL = consts["pitch"], 2 * R * consts["pitch"]
+        planes = (NZ + 1) // 2 * 2
+        first = PL  # X[0], plane 0
+        # the lowest element that a cell reads: the plane below the first, colour 0, beside position 0
+        assert first - PL + 0 * P + 0 >= 0
+        # the highest: the plane above the last, colour 1, last row, beside position 31
+        assert first + planes * PL + R * P + (R - 1) * P + 1 + 32 == x - 1
+        # messages written beside a row: 0 or 33 positions on from the cell beside its first position
+        assert first + (planes - 1) * PL + R * P + (R - 1) * P + 33 < first + planes * PL
+        warps = -(-NZ // (2 * np_))
+        assert warps <= consts["warps"] and warps * np_ * 2 <= planes + 2
+        tail = planes // 2 * 2 * R * 32 * (4 + (16 if bs else 0))
+        assert one == 8 * (x + consts["row"]) + tail
+        # a table row for 600 classes at least, beside the row of the cells without a class
+        rows = (232448 - 512 - (one - 8 * consts["row"])) // (8 * consts["row"])
+        assert rows >= 601, (R, rows)
+    if NZ == 30:
+        # with b in shared memory tiles of 6 rows would have room for 152 classes
+        x, one = sizes[6, 30, 1]
+        assert (232448 - 512 - (one - 80)) // 80 - 1 == 152

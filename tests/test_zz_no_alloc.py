@@ -134,3 +134,27 @@ def test_calcrk_noalloc_calls_from_several_threads(oracle):
         assert got[q] == [alone[q]] * 100
         assert c() == alone[q] and abs(alone[q] - c.res_ref) <= 1e-13 * c.res_ref
         assert np.array_equal(c.residual(), c.r_ref[1:-1, 1:-1, 1:-1])
+
+
+@pytest.mark.parametrize("transient", [False, True], ids=["steady", "transient"])
+@pytest.mark.parametrize("n", [(1, 7, 3), (33, 1, 5), (128, 8, 2), (129, 9, 4), (257, 7, 3), (31, 17, 1), (96, 16, 30)],
+                         ids=lambda n: "x".join(map(str, n)))
+def test_calcrk_noalloc_shapes(oracle, n, transient):
+    """Remainders of the blocks of 8 rows and 128 positions, one cell wide and one row, with five materials, masked
+    cells inside and all boundary types: the oracle's residual to the bit, the norm, and again after a call on a
+    grid with another number of blocks."""
+    from test_gpu_boxes import box_problem
+    prob = box_problem(oracle, *n, seed=sum(n), transient=transient)
+    rng = np.random.default_rng(sum(n))
+    inner = (slice(1, -1),) * 3
+    m = prob.wk["mask"]
+    m[inner] = np.where(rng.uniform(size=m[inner].shape) < 0.1, 0.0, 1.0)
+    prob.wk["theta"][inner] += rng.standard_normal(m[inner].shape)
+    r_ref, res_ref = oracle.calc_rk(prob)
+    call, other = _Call(prob), _Call(mode3_model(oracle, 24, 20))
+    want = other()
+    for _ in range(2):
+        res = call()
+        assert np.array_equal(call.residual(), r_ref[inner])
+        assert abs(res - res_ref) <= 1e-13 * res_ref
+        assert other() == want
