@@ -151,7 +151,7 @@ static __device__ void finish_stage(int stage, SolverState* st, double s1, doubl
 // a/d, the second rounds it correctly.  The remainder is formed negated, so that a zero keeps its
 // sign.  Valid while neither the remainder nor the quotient leaves the normal range: d within
 // 2^+-100 (checked when the class table is made) and a within 2^+-400 or zero; anything else takes the
-// division (div_fix).  5 operations instead of about 39.
+// division (div_fix).
 __device__ __forceinline__ double div_by(double a, double d, double y) {
   double q = __dmul_rn(a, y);
   double r = __fma_rn(d, q, -a);

@@ -14,7 +14,7 @@ const void* pick(int vm) {
 }  // namespace
 
 // One pair of planes a warp: b in shared memory up to 5 rows, from its vector from 6 on (beside x and b of 6
-// rows and 30 planes there is room for 170 classes, and some tiles of the stack have 435); two pairs: b in
+// rows and 30 planes there is room for 152 classes, and some tiles of the stack have 435); two pairs: b in
 // shared memory up to 2 rows.
 const void* resident_kernel(int R, int np, int vm) {
   if (np == 1) {

@@ -40,7 +40,7 @@ constexpr int kRsRowPitch = 34;   // doubles per row in shared memory: 32 positi
 constexpr int kRsBox = 72;        // messages per tile, plane and colour: first row, last row, x edges
 constexpr int kRsZero = 4 * kRsBox;  // slots before the first tile's that nobody writes (zeros)
 constexpr int kRsMaxRows = 8;
-constexpr int kRsMaxWarps = 15;   // 136 registers a thread
+constexpr int kRsMaxWarps = 15;   // 128 registers a thread: four of the warps share a scheduler's 16384
 
 // Number of the next launch (part of every message's pass number), arrivals of the current launch or barrier.
 struct RsCtl {
@@ -87,7 +87,8 @@ __host__ __device__ constexpr size_t rs_smem(int R, int NZ, int ntab, bool bs) {
 }
 
 // One message: 16 bytes, stored and loaded as one (a .b128 access is single-copy atomic).
-// The pass number is 32 bits: every launch writes every slot, so a slot never holds a number 2^32 old.
+// The pass number is 32 bits: 16 for each launch since the messages were cleared, which they are long before it
+// comes round again (resident_prepare).
 __device__ __forceinline__ void msg_store(ulonglong2* p, double v, unsigned seq) {
   asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p),
                "l"(__double_as_longlong(v)), "l"((unsigned long long)seq));

@@ -242,6 +242,7 @@ struct Solver {
   RsCtl* rs_ctl = nullptr;
   ResidentTables rs_tab[kRsMaxRows + 1];  // by rows of a tile
   int rs_rows = 0;              // rows of the tiles whose messages the box holds
+  long long rs_numbers = 0;     // bound of the launches since the box was cleared
   int rs_most = 0;              // dynamic shared memory that the kernels may ask for
   // K right-hand sides on the handle's operator (h2g_create_multi): stacked vectors, K states
   int nrhs = 0;
@@ -477,6 +478,7 @@ static int sweep_status(Solver* s) {
     const RsCtl c{1ull, 0u, 0u};
     CK(cudaMemset(s->rs_box, 0, s->rs_box_cap));
     CK(cudaMemset(s->rs_rowsum, 0, s->rs_rowsum_cap));
+    s->rs_numbers = 0;
     CK(cudaMemcpy(s->rs_ctl, &c, sizeof c, cudaMemcpyHostToDevice));
   }
   CK(cudaStreamSynchronize(cudaStreamLegacy));  // a non-blocking stream does not wait for these by itself
@@ -720,7 +722,7 @@ static bool have(Solver* s, T** p, size_t bytes) {
 // Buffers, the tiles' own class numbers and the shared-memory attributes for the split pl.  pl.R = 0 on
 // return: a tile has more classes than fit beside its x and b, or the device has no memory left for the
 // buffers (the separate passes need none of them).
-static int resident_prepare(Solver* s, ResidentPlan& pl) {
+static int resident_prepare(Solver* s, ResidentPlan& pl, long long launches) {
   const Geo& g = s->g;
   // messages of every split of the grid (a handle may run with all SMs in one call, in fewer and larger tiles,
   // and a share of them in the next) and the guards' rows of k_resident_sor
@@ -746,15 +748,21 @@ static int resident_prepare(Solver* s, ResidentPlan& pl) {
     pl.R = 0;
     return H2G_OK;
   }
-  if (fresh) {
-    const RsCtl init{1ull, 0u, 0u};
-    CK(cudaMemcpyAsync(s->rs_ctl, &init, sizeof init, cudaMemcpyHostToDevice, s->stream));
-    CK(cudaStreamSynchronize(s->stream));
-  } else if (s->rs_rows != pl.R) {
-    // another split writes other slots: none keeps a number from before
+  // No slot may hold a number that comes round again: another split writes other slots and CG no row sums, so the
+  // messages are cleared when the split changes, and with them the count of the launches (28 bits of a pass number)
+  // long before it wraps.
+  const bool count_anew = s->rs_numbers + launches > 1ll << 27;
+  if (!fresh && (count_anew || s->rs_rows != pl.R)) {
     CK(cudaMemsetAsync(s->rs_box, 0, s->rs_box_cap, s->stream));
     CK(cudaMemsetAsync(s->rs_rowsum, 0, s->rs_rowsum_cap, s->stream));
   }
+  if (fresh || count_anew) {
+    const RsCtl init{1ull, 0u, 0u};
+    CK(cudaMemcpyAsync(s->rs_ctl, &init, sizeof init, cudaMemcpyHostToDevice, s->stream));
+    CK(cudaStreamSynchronize(s->stream));
+    s->rs_numbers = 0;
+  }
+  s->rs_numbers += launches;
   s->rs_rows = pl.R;
   if (!t.ntab) {  // the classes were built anew
     std::vector<int> count(pl.blocks());
@@ -2041,12 +2049,12 @@ struct ResidentCall {
   Solver* s = nullptr;
   SmLease lease;
   // The split for one call: within a part of the SMs where other calls are in flight beside it.
-  int plan(Resident what, ResidentPlan& pl) {
+  int plan(Resident what, long long launches, ResidentPlan& pl) {
     pl = resident_plan(s, what, 1);
     if (!pl.R) return H2G_OK;
     const int beside = lease.enter(s);
     if (s->beside > 1 || beside > 1) pl = resident_plan(s, what, s->beside ? s->beside : beside);
-    return pl.R ? resident_prepare(s, pl) : H2G_OK;
+    return pl.R ? resident_prepare(s, pl, launches) : H2G_OK;
   }
   // solveSOR!: the relaxation's quotient by its reciprocal needs omega within 2^+-100 (div_by), and the tiles'
   // set-up takes the time of one to two passes (a call of 1, 2 and 4 passes, us: 40x40x30 57, 67, 82, separate
@@ -2055,7 +2063,7 @@ struct ResidentCall {
     s = solver;
     ResidentPlan pl;
     if (omega >= 0x1p-100 && maxItr > 2)
-      if (int rc = plan(Resident::kSor, pl)) return rc;
+      if (int rc = plan(Resident::kSor, maxItr / 4 + 8ll, pl)) return rc;  // 5 numbers for 32 passes
     if (!pl.R) return H2G_OK;
     CK(cudaFuncSetAttribute(resident_sor_kernel(pl.R, pl.np), cudaFuncAttributeMaxDynamicSharedMemorySize,
                             s->rs_most));
@@ -2063,11 +2071,11 @@ struct ResidentCall {
     s->rs = pl;
     return H2G_OK;
   }
-  int begin(Solver* solver, int smoother, Resident what) {
+  int begin(Solver* solver, int smoother, Resident what, int maxItr) {
     s = solver;
     ResidentPlan pl;
     if (smoother == H2G_SMOOTHER_GS)
-      if (int rc = plan(what, pl)) return rc;
+      if (int rc = plan(what, 2ll * maxItr + 8, pl)) return rc;
     if (pl.R) {
       for (int vm = 0; vm < 3; ++vm)
         CK(cudaFuncSetAttribute(resident_kernel(pl.R, pl.np, vm), cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2095,7 +2103,7 @@ static int solve(Solver* s, bool cg, double tol, int maxItr, int smoother, int v
   if (!(tol >= 0.0) || !std::isfinite(tol)) return fail(H2G_BAD_ARG, "bad tolerance");
   CK(cudaSetDevice(s->device));
   ResidentCall resident;
-  if (int rc = resident.begin(s, smoother, cg ? Resident::kCg : Resident::kPbicgstab)) return rc;
+  if (int rc = resident.begin(s, smoother, cg ? Resident::kCg : Resident::kPbicgstab, maxItr)) return rc;
   int rc;
   if (s->precision == H2G_MIXED_IR) rc = solve_ir(s, cg, tol, maxItr, smoother, verbose, res_hist, out);
   else if (s->precision == H2G_MIXED) rc = solve_mixed(s, cg, tol, maxItr, smoother, verbose, res_hist, out);
@@ -3044,7 +3052,7 @@ static int precond_t(Solver* s, const double* bb, double* xx, int smoother, cons
   void *ha, *hb;
   int rc;
   ResidentCall resident;  // before the hook buffers are filled: the tuner uses them
-  if ((rc = resident.begin(s, smoother, Resident::kPbicgstab))) return rc;
+  if ((rc = resident.begin(s, smoother, Resident::kPbicgstab, 1))) return rc;
   if ((rc = hook_buffers(s, &ha, &hb))) return rc;
   T* xd = static_cast<T*>(ha);
   T* bd = static_cast<T*>(hb);

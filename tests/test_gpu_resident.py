@@ -517,3 +517,25 @@ def test_switches(oracle, monkeypatch):
     s.autotune(), s.sweep(), s.coop()  # asking turns nothing off
     assert forms()
     s.close()
+
+
+def test_messages_are_counted_anew(oracle):
+    """Calls that may take so many iterations that the messages' numbers are counted anew every few of them, with
+    both Krylov methods, SOR and the preconditioner between: always the first call's bits."""
+    prob = mode3_model(oracle, 24, 20)
+    s = make_solver(prob)
+    s.snapshot()
+    bb = random_interior(prob.shape, 3)
+    first = None
+    for _ in range(9):
+        got = []
+        for method in ("pbicgstab", "cg"):
+            s.snapshot(restore=True)
+            st, res = s.solve(method, tol=1e-4, maxItr=10_000_000, smoother="gs")
+            got += [st, res.itr, res.res, s.get_theta()]
+        s.snapshot(restore=True)
+        st, res = s.sor(tol=0.5, maxItr=10_000_000)
+        got += [st, res.itr, res.res, s.get_theta(), s.preconditioner(bb, "gs")]
+        first = first or got
+        assert all(np.array_equal(a, b) for a, b in zip(first, got))
+    s.close()
