@@ -548,13 +548,13 @@ struct SmPool {
     unsigned long long stream;
     bool legacy, blocking, over;
     std::thread::id thread;
-    std::chrono::steady_clock::time_point end;
+    std::chrono::steady_clock::time_point begin, end;
   };
   std::vector<Call> calls;  // in flight (that have their SMs or wait for them), and over for less than kBetween
 };
-// A thread that calls in a loop is between two calls for less than this: without it the threads of a loop find
-// each other missing now and then and change their splits (120x120x30, two threads: 60.8 us an iteration and
-// solve instead of 50.8).
+// A thread that calls in a loop is between two calls for less than this.  A call that is over for no longer, and that
+// the thread's own last call overlapped, counts as one in flight: else the threads of a loop find each other missing
+// now and then and change their splits (120x120x30, two threads: 60.8 us an iteration and solve instead of 50.8).
 constexpr std::chrono::microseconds kBetween(1000);
 constexpr int kMaxDevices = 64;
 static SmPool g_sm_pool[kMaxDevices];
@@ -592,7 +592,10 @@ class SmLease {
     pool_ = &g_sm_pool[s->device];
     std::lock_guard<std::mutex> lk(pool_->mu);
     auto& calls = pool_->calls;
-    const auto now = std::chrono::steady_clock::now();
+    const auto now = me_.begin = std::chrono::steady_clock::now();
+    SmPool::Call last = {};  // the thread's own last call
+    for (const SmPool::Call& c : calls)
+      if (c.over && c.thread == me_.thread) last = c;
     calls.erase(std::remove_if(calls.begin(), calls.end(),
                                [&](const SmPool::Call& c) {
                                  return c.over && (c.thread == me_.thread || now - c.end > kBetween);
@@ -600,7 +603,8 @@ class SmLease {
                 calls.end());
     std::vector<unsigned long long> others;
     for (const SmPool::Call& c : calls)
-      if (c.thread != me_.thread && c.stream != me_.stream && !(c.legacy && me_.blocking) &&
+      if (c.thread != me_.thread && c.stream != me_.stream &&
+          (!c.over || (last.over && c.end > last.begin && c.begin < last.end)) && !(c.legacy && me_.blocking) &&
           !(c.blocking && me_.legacy) && std::find(others.begin(), others.end(), c.stream) == others.end())
         others.push_back(c.stream);
     calls.push_back(me_);
