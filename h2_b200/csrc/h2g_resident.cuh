@@ -840,8 +840,7 @@ __global__ void __launch_bounds__(32 * kRsMaxWarps, 1) k_resident(const __grid_c
       if (VM != 0) load_u(r + 1);
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
-        const unsigned cl = kp[(c * R + r) * 32];
-        if (VM != 0) rs_coef(tab, cl, 16u, cur, cf);  // cxa: x+ (plane 0), x- (plane 1)
+        if (VM != 0) rs_coef(tab, kp[(c * R + r) * 32], 16u, cur, cf);  // cxa: x+ (plane 0), x- (plane 1)
 #pragma unroll
         for (int w = 0; w < 2; ++w) {
           const int o = c ^ 1, cw = c * 2 + w, ow = o * 2 + w;
@@ -854,9 +853,10 @@ __global__ void __launch_bounds__(32 * kRsMaxWarps, 1) k_resident(const __grid_c
             const double dn = w ? xc[o * 2] : x[o * CP - PL], up = w ? x[o * CP + 2 * PL] : xc[o * 2 + 1];
             // cxa multiplies x+ in the first plane and x- in the second
             const double pa = (e != (w != 0)) ? ot : xc[ow], pb = (e != (w != 0)) ? xc[ow] : ot;
-            const double ax =
+            // a cell without a class: 0 - 1 * 0 (a selection instead costs 240x240x30 1.2 % of a solve; the zero is not one
+            // beside an infinity, which ends the solve in this iteration)
+            const double out =
                 sub(rs_sum(cf[w], cf[w].cxa, cf[w].cxb, pa, pb, on[ow], om[ow], up, dn), mul(cf[w].dd, xc[cw]));
-            const double out = (w ? cl >> 16 : cl & 0xffffu) ? ax : 0.0;
             if (in) {
               A.y[ci] = out;
               if (VM == 1) {
