@@ -2061,12 +2061,13 @@ struct ResidentCall {
     return pl.R ? resident_prepare(s, pl, launches) : H2G_OK;
   }
   // solveSOR!: the relaxation's quotient by its reciprocal needs omega within 2^+-100 (div_by), and the tiles'
-  // set-up takes the time of one to two passes (a call of 1, 2 and 4 passes, us: 40x40x30 57, 67, 82, separate
-  // 44, 63, 93; 120x120x30 68, 78, 96, separate 56, 70, 106; 240x240x30 103, 121, 159, separate 85, 120, 185)
+  // set-up takes the time of one to three passes (a call of 1, 2 and 4 passes, us: 40x40x30 57, 67, 82, separate
+  // 44, 63, 93; 240x240x30 103, 121, 159, separate 85, 120, 185; by number of passes, ratio to the separate ones: 98x76x30 3
+  // 1.11, 4 1.04, 5 0.94; 325x54x10 4 1.08, 5 1.01, 6 0.96)
   int begin_sor(Solver* solver, double omega, int maxItr) {
     s = solver;
     ResidentPlan pl;
-    if (omega >= 0x1p-100 && maxItr > 2)
+    if (omega >= 0x1p-100 && maxItr > 5)
       if (int rc = plan(Resident::kSor, maxItr / 4 + 8ll, pl)) return rc;  // 5 numbers for 32 passes
     if (!pl.R) return H2G_OK;
     CK(cudaFuncSetAttribute(resident_sor_kernel(pl.R, pl.np), cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -229,7 +229,7 @@ int h2g_transient(h2g_solver *h, const h2g_bc *bc, int nt, int method, double to
                   int verbose, double *step_stats, h2g_result *out);
 
 /* ---- the form of a solve (no reference counterpart) ----------------------------------------
- * FP64 solves and h2g_preconditioner with the RB-GS smoother, and h2g_sor calls of more than two
+ * FP64 solves and h2g_preconditioner with the RB-GS smoother, and h2g_sor calls of more than five
  * passes, keep their iterate in the SMs' shared memory (k_resident, k_resident_sor) on grids of up to
  * 60 planes that have an SM for every tile and for which that is the faster form; all others run as
  * separate passes.  The results are the same bits.  The form shows in h2g_result.launches: 3 an
