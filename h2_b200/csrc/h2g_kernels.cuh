@@ -1536,7 +1536,7 @@ __global__ void k_make_keys(Geo g, const double* __restrict__ lam, const double*
 
 // ------------------------------------------------------------------------------------------
 // (key, rho*cp) pairs of a transient grid's updated cells.  Pass 1 collects the distinct rho*cp bit
-// patterns like the lambda values; pass 2 marks the pairs key | index << 7 that occur; pass 3 writes
+// patterns like the lambda values; pass 2 marks the pairs key | slot << 7 that occur; pass 3 writes
 // each cell's pair number | 0x80 (numbered by the host; 0 where the cell is never updated).
 // ------------------------------------------------------------------------------------------
 __device__ __forceinline__ int slot_of(const unsigned long long* slots, unsigned long long b) {
@@ -1570,20 +1570,19 @@ __global__ void __launch_bounds__(256) k_collect_rc(Geo g, const uint8_t* __rest
 __global__ void __launch_bounds__(256) k_mark_pairs(Geo g, const uint8_t* __restrict__ key,
                                                      const double* __restrict__ rc,
                                                      const unsigned long long* __restrict__ slots,
-                                                     const int* __restrict__ slot_index, unsigned* bits) {
+                                                     const int* __restrict__ flags, unsigned* bits) {
   const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
   const int j = 1 + blockIdx.y, k = 1 + blockIdx.z;
-  if (i > g.NX) return;
+  if (i > g.NX || *flags) return;
   const int o = g.off(i, j, k);
   if (!(key[o] & 0x80)) return;
-  const int id = (key[o] & 0x7f) | slot_index[slot_of(slots, (unsigned long long)__double_as_longlong(rc[o]))] << 7;
+  const int id = (key[o] & 0x7f) | slot_of(slots, (unsigned long long)__double_as_longlong(rc[o])) << 7;
   if (!(bits[id >> 5] >> (id & 31) & 1u)) atomicOr(bits + (id >> 5), 1u << (id & 31));
 }
 
 __global__ void __launch_bounds__(256) k_write_pairs(Geo g, const uint8_t* __restrict__ key,
                                                       const double* __restrict__ rc,
                                                       const unsigned long long* __restrict__ slots,
-                                                      const int* __restrict__ slot_index,
                                                       const uint8_t* __restrict__ number, uint8_t* __restrict__ pair) {
   const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
   const int j = 1 + blockIdx.y, k = 1 + blockIdx.z;
@@ -1593,7 +1592,7 @@ __global__ void __launch_bounds__(256) k_write_pairs(Geo g, const uint8_t* __res
     pair[o] = 0;
     return;
   }
-  const int id = (key[o] & 0x7f) | slot_index[slot_of(slots, (unsigned long long)__double_as_longlong(rc[o]))] << 7;
+  const int id = (key[o] & 0x7f) | slot_of(slots, (unsigned long long)__double_as_longlong(rc[o])) << 7;
   pair[o] = number[id] | 0x80;
 }
 

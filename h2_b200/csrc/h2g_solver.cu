@@ -1095,30 +1095,18 @@ static int build_pairs(Solver* s, bool* ok) {
   CK(cudaMemsetAsync(s->flags, 0, sizeof(int), s->stream));
   CK(cudaMemsetAsync(s->pair_bits, 0, kIds / 8, s->stream));
   k_collect_rc<<<gi, 256, 0, s->stream>>>(g, s->key, s->rc64, s->slots, s->flags);
+  k_mark_pairs<<<gi, 256, 0, s->stream>>>(g, s->key, s->rc64, s->slots, s->flags, s->pair_bits);
   CKL();
   std::vector<unsigned long long> slots(kHashSlots);
   int flags = 0;
   CK(cudaMemcpyAsync(slots.data(), s->slots, sizeof(unsigned long long) * kHashSlots, cudaMemcpyDeviceToHost, s->stream));
   CK(cudaMemcpyAsync(&flags, s->flags, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+  std::vector<unsigned> bits(kIds / 32);
+  CK(cudaMemcpyAsync(bits.data(), s->pair_bits, kIds / 8, cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));
   s->pairs_ok = false;
   s->pairs_known = true;  // too many values or pairs, unless they turn out to fit
   if (flags) return H2G_OK;
-  std::vector<int> index(kHashSlots, 0);
-  std::vector<double> value;
-  for (int h = 0; h < kHashSlots; ++h)
-    if (slots[h] != ~0ull) {
-      index[h] = (int)value.size();
-      double v;
-      memcpy(&v, &slots[h], sizeof v);
-      value.push_back(v);
-    }
-  CK(cudaMemcpyAsync(s->slot_index, index.data(), sizeof(int) * kHashSlots, cudaMemcpyHostToDevice, s->stream));
-  k_mark_pairs<<<gi, 256, 0, s->stream>>>(g, s->key, s->rc64, s->slots, s->slot_index, s->pair_bits);
-  CKL();
-  std::vector<unsigned> bits(kIds / 32);
-  CK(cudaMemcpyAsync(bits.data(), s->pair_bits, kIds / 8, cudaMemcpyDeviceToHost, s->stream));
-  CK(cudaStreamSynchronize(s->stream));
   std::vector<uint8_t> num(kIds + 128, 0);
   std::vector<double> rc64(128, 0.0);
   std::vector<float> rc32(128, 0.0f);
@@ -1128,14 +1116,14 @@ static int build_pairs(Solver* s, bool* ok) {
     if (n >= kMaxKeys) return H2G_OK;
     num[id] = (uint8_t)n;
     num[kIds + n] = (uint8_t)(id & 0x7f);
-    rc64[n] = value[id >> 7];
-    rc32[n] = (float)value[id >> 7];
+    memcpy(&rc64[n], &slots[id >> 7], sizeof(double));
+    rc32[n] = (float)rc64[n];
     ++n;
   }
   CK(cudaMemcpyAsync(s->pair_num, num.data(), num.size(), cudaMemcpyHostToDevice, s->stream));
   CK(cudaMemcpyAsync(s->pair_rc64, rc64.data(), sizeof(double) * 128, cudaMemcpyHostToDevice, s->stream));
   CK(cudaMemcpyAsync(s->pair_rc32, rc32.data(), sizeof(float) * 128, cudaMemcpyHostToDevice, s->stream));
-  k_write_pairs<<<gi, 256, 0, s->stream>>>(g, s->key, s->rc64, s->slots, s->slot_index, s->pair_num, s->pair);
+  k_write_pairs<<<gi, 256, 0, s->stream>>>(g, s->key, s->rc64, s->slots, s->pair_num, s->pair);
   CKL();
   CK(cudaStreamSynchronize(s->stream));  // the host vectors must outlive the copies
   *ok = s->pairs_ok = n > 0;
